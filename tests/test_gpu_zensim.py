@@ -71,3 +71,23 @@ def test_zensim_errors(tmb, cuda):
     img = cuda.zeros((64, 65, 3), dtype=cuda.uint8, device="cuda")
     assert z.mem_usage() > 0
     z.close()
+
+
+@pytest.mark.parametrize("w,h", [(8, 8), (16, 9), (17, 40), (33, 31), (63, 64), (65, 33), (130, 97), (529, 70), (40, 200)])
+def test_zensim_at_tile_and_chunk_edges(tmb, oracle, cuda, w, h):
+    """Sizes around the feature tile (64 x 32), the saved states (every 8
+    rows), the walk's chunks (32 rows) and blocks (32 columns) and the padded
+    width; the images are crops whose rows start at odd addresses."""
+    ref, dis = synth.srgb_pair(w + 1, h, 78, 12)
+    crop = [dev(cuda, a)[:, 1:] for a in (ref, dis)]
+    ref, dis = (np.ascontiguousarray(a[:, 1:]) for a in (ref, dis))
+    z = tmb.Zensim(w, h)
+    feat = z.compute_features(*crop)
+    acc, peaks = z.raw()
+    want = oracle.zensim_features_srgb8(ref, dis)
+    ns = want.n_scales
+    assert z.n_scales == ns
+    assert np.array_equal(peaks[:ns], want.peaks[:ns])
+    np.testing.assert_allclose(acc[:ns], want.acc[:ns], rtol=1e-9, atol=1e-12)
+    np.testing.assert_allclose(feat, want.features, rtol=1e-9, atol=1e-12)
+    z.close()

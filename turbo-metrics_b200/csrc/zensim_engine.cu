@@ -2,14 +2,14 @@
 // Zensim::new / set_reference / compute_with_reference / compute_features /
 // has_reference / clear_reference / debug_compute_raw of crates/zensim-cuda
 // (src/lib.rs:168-819).  The reference's XYB pyramid stays resident after
-// set_reference; every compute converts the distorted image, builds its
-// pyramid, runs one feature launch over all (scale, channel, strip) items and
-// forms the 228 features on the host from the fixed-order sums.
+// set_reference; every compute converts the distorted image and its pyramid
+// (one launch), walks the vertical sums, scores the tiles and reduces them
+// (three launches), and forms the 228 features on the host from the sums of
+// each (scale, channel).
 #include <cuda_runtime.h>
 
 #include <cmath>
 #include <cstring>
-#include <vector>
 
 #include "../../include/ssim2b200.h"
 #include "zensim_kernels.h"
@@ -36,24 +36,39 @@ int simd_padded_width(int w) {
     return (aligned >= 512 && (aligned / 16) % 2 == 0) ? aligned + 16 : aligned;
 }
 
+// cbrtf_fast of the opsin bias, negated, with the device's operations (this
+// unit's host code is built with -ffp-contract=off)
+float opsin_bias() {
+    const float x = 0.0037930734f;
+    uint32_t u;
+    std::memcpy(&u, &x, 4);
+    u = u / 3u + 709958130u;
+    float t;
+    std::memcpy(&t, &u, 4);
+    for (int k = 0; k < 2; k++) {
+        const float r = t * t * t;
+        t = t * (std::fmaf(x, 2.0f, r) / std::fmaf(r, 2.0f, x));
+    }
+    return -t;
+}
+
 }  // namespace
 
 struct s2_zensim {
     int device = 0;
     uint32_t w = 0, h = 0;
-    int ns = 0;
-    int n[kZsScales] = {0, 0, 0, 0}, hh[kZsScales] = {0, 0, 0, 0};
-    ZsScale sc[kZsScales];
-    void *planes = nullptr;      // both pyramids
-    uint8_t *stage = nullptr;    // device copy of host inputs (w * 3 * h bytes)
-    ZsScale *sc_d = nullptr;     // scale descriptors
-    ZsItem *items_d = nullptr;   // work items
-    double *out_d = nullptr;     // kZsOut doubles per item
-    std::vector<ZsItem> items;
-    std::vector<double> out_h;
+    ZsPlan plan = {};
+    void *planes = nullptr;       // both pyramids, then the saved states of the vertical sums
+    size_t plane_bytes = 0;
+    uint8_t *stage = nullptr;     // device copy of host inputs (w * 3 * h bytes)
+    double *tile_out = nullptr;   // kZsOut doubles per tile, then per (scale, channel)
+    double out_h[kZsScales * 3 * kZsOut];  // host copy of the latter
     bool has_ref = false;
     double raw_acc[kZsScales][3][kZsSums];
     uint32_t raw_peak[kZsScales][3][3];
+
+    size_t out_doubles() const { return (size_t)kZsOut * 3 * plan.ns; }
+    size_t tile_doubles() const { return (size_t)kZsOut * plan.tiles; }
 };
 
 static bool g_zs_lut_ready[64];
@@ -66,6 +81,7 @@ s2_status s2_zensim_create(int32_t device, uint32_t width, uint32_t height, s2_z
     ZS_CUDA(cudaSetDevice(device));
     if (device >= 0 && device < 64 && !g_zs_lut_ready[device]) {
         ZS_CUDA(zs_upload_lut(s2_srgb8_lut));
+        ZS_CUDA(zs_configure());
         g_zs_lut_ready[device] = true;
     }
     s2_zensim *z = new s2_zensim();
@@ -75,53 +91,49 @@ s2_status s2_zensim_create(int32_t device, uint32_t width, uint32_t height, s2_z
     z->w = width;
     z->h = height;
     // scales while the logical width and the height are >= 8 (lib.rs:222-233)
+    ZsPlan &P = z->plan;
     int lw = (int)width, n = simd_padded_width((int)width), h = (int)height;
-    size_t bytes = 0, off[kZsScales][2];
+    size_t bytes = 0, off[kZsScales][2], state[kZsScales];
     for (int s = 0; s < kZsScales; s++) {
         if (lw < 8 || h < 8) break;
-        z->n[s] = n;
-        z->hh[s] = h;
-        const size_t pitch = align_up((size_t)n, 64);
+        ZsScale &S = P.sc[s];
+        S.n = S.ref.n = S.dis.n = n;
+        S.h = h;
+        S.ref.pitch = S.dis.pitch = align_up((size_t)(kZsLeft + n + kZsRight), 64);
         for (int img = 0; img < 2; img++) {
             off[s][img] = bytes;
-            bytes += 3 * align_up(pitch * h * sizeof(float), 256);
+            bytes += 3 * align_up(S.ref.pitch * h * sizeof(float), 256);
         }
-        z->ns++;
+        state[s] = bytes;
+        bytes += align_up((size_t)3 * ((h + kZsSub - 1) / kZsSub) * 4 * S.ref.pitch * sizeof(float), 256);
+        S.walk_x = (n + kZsWalkW - 1) / kZsWalkW;
+        S.walk_first = P.walk_blocks;
+        P.walk_blocks += 3 * S.walk_x;
+        S.tiles_x = (n + kZsTileW - 1) / kZsTileW;
+        S.tiles_y = (h + kZsTileH - 1) / kZsTileH;
+        S.tile_first = P.tiles;
+        P.tiles += 3 * S.tiles_x * S.tiles_y;
+        P.ns++;
         lw = (lw + 1) / 2;
         n = n / 2;
         h = (h + 1) / 2;
     }
-    for (int s = 0; s < z->ns; s++)
-        for (int c = 0; c < 3; c++)
-            for (int x0 = 0; x0 < z->n[s]; x0 += kZsCols) z->items.push_back(ZsItem{s, c, x0});
-    z->out_h.resize(z->items.size() * kZsOut);
+    z->plane_bytes = bytes;
     cudaError_t e = cudaMalloc(&z->planes, bytes);
     if (e == cudaSuccess) e = cudaMalloc((void **)&z->stage, (size_t)width * 3 * height);
-    if (e == cudaSuccess) e = cudaMalloc((void **)&z->sc_d, sizeof(ZsScale) * kZsScales);
-    if (e == cudaSuccess) e = cudaMalloc((void **)&z->items_d, sizeof(ZsItem) * z->items.size());
-    if (e == cudaSuccess) e = cudaMalloc((void **)&z->out_d, sizeof(double) * z->out_h.size());
+    if (e == cudaSuccess)
+        e = cudaMalloc((void **)&z->tile_out, sizeof(double) * (z->tile_doubles() + z->out_doubles()));
     if (e != cudaSuccess) {
         s2_zensim_destroy(z);
         return e == cudaErrorMemoryAllocation ? S2_ERR_OOM : s2_cuda_fail(e, "zensim buffers");
     }
-    for (int s = 0; s < z->ns; s++) {
-        const size_t pitch = align_up((size_t)z->n[s], 64);
-        const size_t plane = align_up(pitch * z->hh[s] * sizeof(float), 256);
-        ZsPlanes *pl[2] = {&z->sc[s].ref, &z->sc[s].dis};
-        for (int img = 0; img < 2; img++) {
-            for (int c = 0; c < 3; c++) pl[img]->p[c] = (float *)((char *)z->planes + off[s][img] + c * plane);
-            pl[img]->n = z->n[s];
-            pl[img]->pitch = pitch;
-        }
-        z->sc[s].n = z->n[s];
-        z->sc[s].h = z->hh[s];
-    }
-    e = cudaMemcpy(z->sc_d, z->sc, sizeof(ZsScale) * kZsScales, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess)
-        e = cudaMemcpy(z->items_d, z->items.data(), sizeof(ZsItem) * z->items.size(), cudaMemcpyHostToDevice);
-    if (e != cudaSuccess) {
-        s2_zensim_destroy(z);
-        return s2_cuda_fail(e, "zensim descriptors");
+    for (int s = 0; s < P.ns; s++) {
+        ZsScale &S = P.sc[s];
+        const size_t plane = align_up(S.ref.pitch * S.h * sizeof(float), 256);
+        ZsPlanes *pl[2] = {&S.ref, &S.dis};
+        for (int img = 0; img < 2; img++)
+            for (int c = 0; c < 3; c++) pl[img]->p[c] = (float *)((char *)z->planes + off[s][img] + c * plane) + kZsLeft;
+        S.state = (float *)((char *)z->planes + state[s]);
     }
     *out = z;
     return S2_OK;
@@ -133,9 +145,7 @@ void s2_zensim_destroy(s2_zensim *z) {
     cudaDeviceSynchronize();
     cudaFree(z->planes);
     cudaFree(z->stage);
-    cudaFree(z->sc_d);
-    cudaFree(z->items_d);
-    cudaFree(z->out_d);
+    cudaFree(z->tile_out);
     delete z;
 }
 
@@ -150,10 +160,8 @@ static s2_status zs_pyramid(s2_zensim *z, int img, const uint8_t *src, size_t pi
         src = z->stage;
         pitch = row;
     }
-    ZsPlanes ZsScale::*which = img ? &ZsScale::dis : &ZsScale::ref;
-    ZS_CUDA(zs_launch_xyb(src, pitch, (int)z->w, (int)z->h, z->sc[0].*which, st));
-    for (int s = 1; s < z->ns; s++)
-        ZS_CUDA(zs_launch_down(z->sc[s - 1].*which, z->hh[s - 1], z->sc[s].*which, z->hh[s], st));
+    static const float bias = opsin_bias();
+    ZS_CUDA(zs_launch_prep(src, pitch, (int)z->w, (int)z->h, z->plan, img, bias, st));
     return S2_OK;
 }
 
@@ -173,9 +181,9 @@ s2_status s2_zensim_set_reference_srgb8(s2_zensim *z, const uint8_t *ref, size_t
 // lib.rs:686-819: the 228 features from the sums of each (scale, channel)
 static void zs_assemble(s2_zensim *z, double *feat) {
     std::memset(feat, 0, sizeof(double) * kZsFeatures);
-    const int basic_total = z->ns * 13 * 3;
-    for (int s = 0; s < z->ns; s++) {
-        const double inv_n = 1.0 / ((double)z->n[s] * (double)z->hh[s]);
+    const int basic_total = z->plan.ns * 13 * 3;
+    for (int s = 0; s < z->plan.ns; s++) {
+        const double inv_n = 1.0 / ((double)z->plan.sc[s].n * (double)z->plan.sc[s].h);
         for (int c = 0; c < 3; c++) {
             const double *r = z->raw_acc[s][c];
             const uint32_t *pk = z->raw_peak[s][c];
@@ -216,24 +224,23 @@ s2_status s2_zensim_compute_with_reference_srgb8(s2_zensim *z, const uint8_t *di
     cudaStream_t st = (cudaStream_t)stream;
     s2_status r = zs_pyramid(z, 1, dis, pitch, on_host, st);
     if (r != S2_OK) return r;
-    ZS_CUDA(zs_launch_feat(z->sc_d, z->items_d, (int)z->items.size(), z->out_d, st));
-    ZS_CUDA(cudaMemcpyAsync(z->out_h.data(), z->out_d, sizeof(double) * z->out_h.size(), cudaMemcpyDeviceToHost,
-                            st));
+    double *const out_d = z->tile_out + z->tile_doubles();
+    ZS_CUDA(zs_launch_features(z->plan, z->tile_out, out_d, st));
+    ZS_CUDA(cudaMemcpyAsync(z->out_h, out_d, sizeof(double) * z->out_doubles(), cudaMemcpyDeviceToHost, st));
     ZS_CUDA(cudaStreamSynchronize(st));
-    // items are ordered (scale, channel, strip): strips added left to right
     std::memset(z->raw_acc, 0, sizeof z->raw_acc);
-    float peak[kZsScales][3][3] = {};
-    for (size_t i = 0; i < z->items.size(); i++) {
-        const ZsItem &it = z->items[i];
-        const double *o = &z->out_h[i * kZsOut];
-        for (int k = 0; k < kZsSums; k++) z->raw_acc[it.scale][it.ch][k] += o[k];
-        for (int k = 0; k < 3; k++) peak[it.scale][it.ch][k] = std::fmax(peak[it.scale][it.ch][k], (float)o[kZsSums + k]);
-    }
-    for (int s = 0; s < kZsScales; s++)
-        for (int c = 0; c < 3; c++)
-            for (int k = 0; k < 3; k++) std::memcpy(&z->raw_peak[s][c][k], &peak[s][c][k], 4);
+    std::memset(z->raw_peak, 0, sizeof z->raw_peak);
+    for (int s = 0; s < z->plan.ns; s++)
+        for (int c = 0; c < 3; c++) {
+            const double *o = z->out_h + (size_t)kZsOut * (3 * s + c);
+            std::memcpy(z->raw_acc[s][c], o, sizeof(double) * kZsSums);
+            for (int k = 0; k < 3; k++) {
+                const float peak = (float)o[kZsSums + k];
+                std::memcpy(&z->raw_peak[s][c][k], &peak, 4);
+            }
+        }
     zs_assemble(z, features);
-    if (n_scales) *n_scales = z->ns;
+    if (n_scales) *n_scales = z->plan.ns;
     return S2_OK;
 }
 
@@ -262,10 +269,8 @@ s2_status s2_zensim_raw(const s2_zensim *z, double *acc, uint32_t *peaks) {
 
 s2_status s2_zensim_mem_usage(const s2_zensim *z, size_t *bytes) {
     if (!z || !bytes) return S2_ERR_INVALID_ARG;
-    size_t b = (size_t)z->w * 3 * z->h + sizeof(ZsScale) * kZsScales + sizeof(ZsItem) * z->items.size() +
-               sizeof(double) * z->out_h.size();
-    for (int s = 0; s < z->ns; s++)
-        b += 6 * align_up(align_up((size_t)z->n[s], 64) * z->hh[s] * sizeof(float), 256);
+    const size_t b = (size_t)z->w * 3 * z->h + z->plane_bytes +
+                     sizeof(double) * (z->tile_doubles() + z->out_doubles());
     *bytes = b;
     return S2_OK;
 }
