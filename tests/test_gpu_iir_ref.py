@@ -58,3 +58,17 @@ def test_iir_ref_differs_from_fir_as_the_reference_does(tmb, oracle, cuda):
     exact = oracle.ssim2_srgb8(ref, dis, "fp64").score
     assert abs(out["fir"] - exact) < 1e-4
     assert abs(out["iir_ref"] - exact) > 1e-3
+
+
+@pytest.mark.parametrize("w,h", [(8, 8), (28, 12), (29, 28), (32, 32), (33, 31), (61, 44), (92, 27), (64, 13), (60, 65)])
+def test_iir_ref_at_chunk_edges(tmb, oracle, cuda, w, h):
+    """Lines around the walks' chunks (16 rows, 32 columns; the walk runs 4
+    samples past the line) and row groups (32 rows)."""
+    ref, dis = synth.srgb_pair(w, h, 91, 12)
+    s = tmb.Ssimulacra2(w, h, blur="iir_ref", scale_rule="all6")
+    s.compute_srgb(cuda.from_numpy(ref).cuda(), cuda.from_numpy(dis).cuda())
+    score, stats, _ = s.get_result()
+    mirror = oracle.ssim2_srgb8(ref, dis, "cuda32", "all6")
+    ok, bad = close(stats, mirror.stats)
+    assert ok, (bad, stats[bad], mirror.stats[bad])
+    assert abs(score - mirror.score) < 1e-6

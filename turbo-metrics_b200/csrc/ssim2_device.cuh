@@ -103,10 +103,10 @@ struct Seg {
     int strip_rows;
 };
 
-// A run of S2_BLUR_IIR_REF work items of one (pair, scale): columns x planes
-// for the vertical walk, rows x channels for the horizontal walk.
+// A run of S2_BLUR_IIR_REF blocks of one (pair, scale): one per (32 columns,
+// channel) of the vertical walk, one per (32 rows, channel) of the horizontal.
 struct IirSeg {
-    int first;     // first work item
+    int first;     // first block
     int pair;
     int scale;
     int rec_base;  // first row record of this (pair, scale) in the partial sums

@@ -557,8 +557,8 @@ struct Engine {
         if (blur == S2_BLUR_IIR_REF) {
             P.grp_pair = {0, n};
             P.grp_tile = {0, 0};
-            // one partial-sum record per row; vertical work items per column
-            // (groups of 32) and plane, horizontal per row and channel
+            // one partial-sum record per row; vertical blocks per 32
+            // columns and channel, horizontal blocks per 32 rows and channel
             int rec = 0;
             for (int i = 0; i < n; i++) {
                 DevPair &p = P.pairs[i];
@@ -572,11 +572,11 @@ struct Engine {
                     v.rec_base = rec;
                     v.v = (float *)P.v_bytes;  // offset, rebased at upload
                     P.vsegs.push_back(v);
-                    P.vtotal += ((p.w[s] + 31) / 32) * 32 * 15;
+                    P.vtotal += 3 * ((p.w[s] + 31) / 32);
                     IirSeg h = v;
                     h.first = P.htotal;
                     P.hsegs.push_back(h);
-                    P.htotal += 3 * p.h[s];
+                    P.htotal += 3 * ((p.h[s] + 31) / 32);
                     p.tile_base[s] = rec;
                     p.tile_cnt[s] = p.h[s];
                     rec += p.h[s];

@@ -986,6 +986,7 @@ cudaError_t configure_kernels() {
     cudaError_t e;
     if ((e = fused_attrs<false>()) != cudaSuccess) return e;
     if ((e = fused_attrs<true>()) != cudaSuccess) return e;
+    if ((e = configure_iir_kernels()) != cudaSuccess) return e;
     return configure_dssim_kernels();
 }
 

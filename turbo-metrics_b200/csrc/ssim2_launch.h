@@ -32,6 +32,8 @@ TileCheck tile_check(int *err);  // the process-wide setting (s2_debug_tile_time
 cudaError_t launch_fused(int storage, const DevPair *pairs, const Seg *segs, int nseg, int first_tile,
                          int end_tile, int *counter, const TileCheck &ck, double *partials, int grid,
                          cudaStream_t st);
+// vtotal, htotal: blocks of the vertical and the horizontal walk
+cudaError_t configure_iir_kernels();
 cudaError_t launch_iir(int storage, const DevPair *pairs, const IirSeg *vsegs, int nvseg, int vtotal,
                        const IirSeg *hsegs, int nhseg, int htotal, double *partials, cudaStream_t st);
 // Copy `bytes` (a multiple of 16, both pointers 16-byte aligned) from
