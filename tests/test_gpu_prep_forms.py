@@ -1,0 +1,42 @@
+"""The prep pass's two block forms (32 x 32 pixels of one image for few blocks,
+64 x 64 of both images beyond two per SM) write the same planes: a pair alone
+(small form) and the same pair in a batch large enough for the large form give
+the same statistics, bit for bit at a fixed tile height, in every input format
+and with DSSIM's planes from the same pass."""
+import numpy as np
+import pytest
+
+import synth
+
+pytestmark = pytest.mark.gpu
+
+
+def _pair(tmb, cuda, fmt, w, h):
+    d = lambda a: cuda.from_numpy(np.ascontiguousarray(a)).cuda()
+    rng = np.random.RandomState(w + h)
+    if fmt in ("nv12", "p016"):
+        (ry, ruv), (dy, duv) = synth.nv12_frame_pair(w, h, 31)
+        if fmt == "p016":
+            ry, ruv, dy, duv = (a.astype(np.int16) << 7 for a in (ry, ruv, dy, duv))
+        return tmb.PairDesc(d(ry), d(dy), fmt, d(ruv), d(duv))
+    ref, dis = synth.srgb_pair(w, h, 32, 12)
+    if fmt == "rgb16":
+        ref, dis = (a.astype(np.int16) * 4 + rng.randint(0, 4, a.shape).astype(np.int16) for a in (ref, dis))
+    if fmt == "linear_f32":
+        ref, dis = ((a / np.float32(255)) ** np.float32(2) for a in (ref, dis))
+    return tmb.PairDesc(d(ref), d(dis), fmt)
+
+
+@pytest.mark.parametrize("fmt", ["srgb8", "nv12", "p016", "rgb16", "linear_f32"])
+@pytest.mark.parametrize("w,h", [(8, 8), (32, 34), (62, 66), (130, 98), (200, 150)])
+def test_small_and_large_blocks_agree(tmb, cuda, fmt, w, h):
+    odd = 0 if fmt in ("nv12", "p016") else 1
+    p = _pair(tmb, cuda, fmt, w + odd, h + odd)
+    big = _pair(tmb, cuda, fmt, 1024, 1280)  # 320 large blocks
+    b = tmb.Ssim2Batch(2, 4 << 20, strip_rows=32)
+    b.set_metrics(("ssimulacra2", "dssim"))
+    alone = b.compute_batch([p])[0]
+    both = b.compute_batch([p, big])[0]
+    assert alone[0] == both[0] and alone[5] == both[5]
+    for k in (1, 2, 6):
+        assert np.array_equal(alone[k], both[k])

@@ -21,7 +21,8 @@ constexpr int kStep = 8;             // output rows per vertical / horizontal st
 constexpr int kSegW = 8;             // output pixels per horizontal task (one f32 partial sum)
 constexpr int kSegs = kTileW / kSegW;  // horizontal tasks per row (15)
 constexpr int kStripMin = 16, kStripMid = 32, kStripMax = 64;  // tile heights (divide kBand)
-constexpr int kPyrBlk = 64;          // scale-0 block edge of the prep kernel
+constexpr int kPyrBlk = 64;          // scale-0 block edge of the prep kernel, ...
+constexpr int kPyrBlkSmall = 32;     // ... and of its form for few blocks (multiples of 2^5)
 constexpr float kC2 = 0.0009f;
 constexpr int kDsLevels = 5;         // DSSIM scales (dssim-cuda/src/lib.rs:73)
 
@@ -50,7 +51,7 @@ struct DevPair {
     int tile_base[kScales];  // first global tile of each scale
     int tile_cnt[kScales];
     int blk_base;            // first pyramid block
-    int blk_x, blk_y;        // pyramid blocks of this pair
+    int blk_x, blk_y;        // pyramid blocks of this pair (of the submission's block edge)
     int status;
     int prep_mask;           // images the prep pass converts: bit 0 reference, bit 1 distorted
     // 4:2:0 YUV (NV12 / P016): y_coeff, r_coeff, b_coeff, g_coeff1, g_coeff2

@@ -126,6 +126,7 @@ struct Plan {
     std::vector<int> blk_first;
     std::vector<Seg> segs;
     int total_blocks = 0;
+    int pyr_blk = kPyrBlk;   // edge of the prep blocks
     int total_tiles = 0;
     size_t level_bytes = 0;  // both images, all levels, all pairs
     int strip_rows = 63;
@@ -442,6 +443,18 @@ struct Engine {
         return off;
     }
 
+    // Edge of the prep blocks.  Up to two 64 x 64 blocks per SM the pass takes
+    // one block's time, and the small form's is shorter; beyond that its blocks
+    // run in waves.  sRGB8 pairs on 148 SMs, small against large form: 640x480
+    // (80 blocks) 12.9 / 23.2 us, 1280x720 (240) 23.5 / 25.9, 1600x1066 (425)
+    // 39.5 / 30.5, 1920x1080 (510) 45.5 / 37.3.
+    int choose_pyr_blk(const s2_pair_desc *d, int n) const {
+        uint64_t blocks = 0;
+        for (int i = 0; i < n; i++)
+            blocks += (uint64_t)((d[i].width + kPyrBlk - 1) / kPyrBlk) * ((d[i].height + kPyrBlk - 1) / kPyrBlk);
+        return blocks <= 2 * (uint64_t)num_sms ? kPyrBlkSmall : kPyrBlk;
+    }
+
     // Lay out the levels and tiles of n pairs.
     s2_status plan(const s2_pair_desc *d, int n, Plan &P, const PairExtra *ex = nullptr, int ngroups = 1) {
         P = Plan();
@@ -464,6 +477,7 @@ struct Engine {
             }
         }
         P.strip_rows = choose_strip_rows(tiles_at, P);
+        P.pyr_blk = choose_pyr_blk(d, n);
         size_t lvl_off = 0;
         int blk = 0;
         for (int i = 0; i < n; i++) {
@@ -525,8 +539,8 @@ struct Engine {
             if (m_ds) lvl_off = plan_dssim(q, p, P.ds[i], lvl_off, ex ? &ex[i] : nullptr, P.ds_clamp);
             P.blk_first[i] = blk;
             {
-                p.blk_x = (p.w[0] + kPyrBlk - 1) / kPyrBlk;
-                p.blk_y = (p.h[0] + kPyrBlk - 1) / kPyrBlk;
+                p.blk_x = (p.w[0] + P.pyr_blk - 1) / P.pyr_blk;
+                p.blk_y = (p.h[0] + P.pyr_blk - 1) / P.pyr_blk;
                 p.blk_base = blk;
                 blk += p.blk_x * p.blk_y;
             }
@@ -765,7 +779,8 @@ struct Engine {
         const Seg *dsegs = (const Seg *)(dbase + pb + bb);
         const int pout = (m_s2 ? 1 : 0) | (m_ds ? 2 : 0);
         if (graphs && !host && !profiling && ng == 1) {
-            const uint64_t key[8] = {(uint64_t)n | ((uint64_t)(uniform_fmt(P) + 1) << 40), (uint64_t)P.total_blocks,
+            const uint64_t key[8] = {(uint64_t)n | ((uint64_t)(uniform_fmt(P) + 1) << 40),
+                                     (uint64_t)P.total_blocks | ((uint64_t)P.pyr_blk << 40),
                                      (uint64_t)P.total_tiles,
                                      P.segs.size(),
                                      P.vsegs.size(), P.hsegs.size(),
@@ -827,7 +842,7 @@ struct Engine {
             const int b0 = pa < n ? P.blk_first[pa] : P.total_blocks;
             const int b1 = pe < n ? P.blk_first[pe] : P.total_blocks;
             S2_CUDA(launch_pyramid(storage, dpairs, n, dblk, b0, b1, cc, (const float *)lut_d.p, num_sms * 8, pst,
-                                   pout, uniform_fmt(P)));
+                                   pout, uniform_fmt(P), P.pyr_blk));
             if (host && g + 1 == ng) S2_CUDA(cudaEventRecord(stage_free, pst));
             if (split) {
                 S2_CUDA(cudaEventRecord(grp_prepped[g], prep_st));
@@ -901,7 +916,7 @@ struct Engine {
         if (e == cudaSuccess)
             e = launch_pyramid(storage, dpairs, n, (const int *)(dbase + pb), 0, P.total_blocks, cc,
                                (const float *)lut_d.p, num_sms * 8, cap_st, (m_s2 ? 1 : 0) | (m_ds ? 2 : 0),
-                               uniform_fmt(P));
+                               uniform_fmt(P), P.pyr_blk);
         if (e == cudaSuccess && m_s2) {
             if (blur == S2_BLUR_IIR_REF)
                 e = launch_iir(storage, dpairs, (const IirSeg *)(dbase + pb + bb + sb), (int)P.vsegs.size(), P.vtotal,

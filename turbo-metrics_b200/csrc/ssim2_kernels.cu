@@ -130,8 +130,6 @@ __device__ __forceinline__ void store_xyb_pair(ST *dst, long long plane, long lo
     }
 }
 
-constexpr int kLv1 = kPyrBlk / 2;  // scale-1 block edge (32)
-
 // DSSIM outputs of one level's pixel: its Lab (levels below lab_levels) and,
 // for the clamp pass, its linear RGB (level lab_levels - 1, when kept).
 __device__ __forceinline__ void store_lab(const DevPair &P, int img, int s, int x, int y, const float lin[3]) {
@@ -184,9 +182,15 @@ __device__ __forceinline__ void store_lab_pair(const DevPair &P, int img, int s,
 // A thread takes two horizontally adjacent 2x2 quads at a time (4 x 2
 // scale-0 pixels): the scale-0 XYB goes out as pixel pairs, and the two
 // quads' scale-1 pixels form one pair for the f32x2 XYB conversion too.
-template <int FMT, typename ST, int OUT>
+//
+// BLK: the block's edge.  A block of kPyrBlk converts both images; one of
+// kPyrBlkSmall converts `only` one.
+template <int FMT, typename ST, int OUT, int BLK>
 __device__ __forceinline__ void prep_quads(const DevPair &P, int X0, int Y0, const float *lut, const ColorConsts &cc,
-                                           float (*lv1)[3][kLv1 * kLv1]) {
+                                           float (*lv1)[3][BLK / 2 * (BLK / 2)], int only) {
+    constexpr int kLv1 = BLK / 2;  // scale-1 block edge
+    constexpr bool kOne = BLK == kPyrBlkSmall;
+    const int mask = kOne ? 1 << only : P.prep_mask;
     constexpr bool KU = FMT != FMT_LINEAR_F32;
     constexpr bool kX = (OUT & 1) != 0, kL = (OUT & 2) != 0;
     constexpr bool kYuv = FMT == FMT_NV12 || FMT == FMT_P016;
@@ -202,18 +206,18 @@ __device__ __forceinline__ void prep_quads(const DevPair &P, int X0, int Y0, con
         // 4:2:0 YUV: both images' samples are loaded before either is converted
         Nv12Quad nr0{}, nr1{}, nd0{}, nd1{};  // [reference, distorted][quad]
         if (kYuv) {
-            if (P.prep_mask & 1) {
+            if (mask & 1) {
                 nr0 = yuv_load_quad<kEs>(P, 0, x, y);
                 if (two) nr1 = yuv_load_quad<kEs>(P, 0, x + 2, y);
             }
-            if (P.prep_mask & 2) {
+            if (mask & 2) {
                 nd0 = yuv_load_quad<kEs>(P, 1, x, y);
                 if (two) nd1 = yuv_load_quad<kEs>(P, 1, x + 2, y);
             }
         }
 #pragma unroll 1
-        for (int img = 0; img < 2; img++) {
-            if (!((P.prep_mask >> img) & 1)) continue;
+        for (int img = kOne ? only : 0; img < (kOne ? only + 1 : 2); img++) {
+            if (!kOne && !((mask >> img) & 1)) continue;
             float l1[2][3];
 #pragma unroll
             for (int k = 0; k < 2; k++) {
@@ -256,8 +260,8 @@ __device__ __forceinline__ void prep_quads(const DevPair &P, int X0, int Y0, con
             const int x1 = (X0 >> 1) + qx, y1 = (Y0 >> 1) + qy;
 #pragma unroll
             for (int c = 0; c < 3; c++) {
-                lv1[img][c][qy * kLv1 + qx] = l1[0][c];
-                if (two) lv1[img][c][qy * kLv1 + qx + 1] = l1[1][c];
+                lv1[kOne ? 0 : img][c][qy * kLv1 + qx] = l1[0][c];
+                if (two) lv1[kOne ? 0 : img][c][qy * kLv1 + qx + 1] = l1[1][c];
             }
             if (kX && (!kL || P.nscales > 1)) {
                 // x1 is even and the planes' pitch a multiple of 64 elements
@@ -278,13 +282,22 @@ constexpr int kPrepThreads = 128;
 // block then switches on its pair's format).  A kernel compiled for one
 // format carries one conversion instead of five, which the instruction
 // cache notices.
-template <typename ST, int OUT, int FMT>
+//
+// BLK kPyrBlkSmall: blocks of 32 x 32 pixels of one image, one step of
+// two quads per thread where the 64 x 64 form takes four steps of two images
+// one after the other.  Its levels below the second keep a few threads busy
+// and it fetches a descriptor per 1,024 pixels, so the 64 x 64 form has the
+// better rate once its blocks fill the SMs: a 96x64 pair 10.5 us instead of
+// 22.1 (latencies), but 3840x2160 162 instead of 115.
+template <typename ST, int OUT, int FMT, int BLK>
 __global__ void __launch_bounds__(kPrepThreads, 4) prep_kernel(const DevPair *__restrict__ pairs, int npairs,
                                                    const int *__restrict__ blk_first, int first_block,
                                                    int end_block,
                                                    ColorConsts cc, const float *__restrict__ lut_g) {
-    __shared__ float lv1[2][3][kLv1 * kLv1];              // scale-1 linear block [img][ch][px]
-    __shared__ float pp[2][2][3][(kLv1 / 2) * (kLv1 / 2)];  // scales >= 2, ping-pong
+    constexpr int kLv1 = BLK / 2;
+    constexpr int kImgs = BLK == kPyrBlkSmall ? 1 : 2;        // images of a block
+    __shared__ float lv1[kImgs][3][kLv1 * kLv1];              // scale-1 linear block [img][ch][px]
+    __shared__ float pp[2][kImgs][3][(kLv1 / 2) * (kLv1 / 2)];  // scales >= 2, ping-pong
     __shared__ float lut[256 + 4];  // the sRGB8 table, then the BT.709 power's 2^(20e/9) factors
     // the block's pair descriptor: in shared memory, so the level stores
     // (global) cannot alias it and its fields need no per-thread copy
@@ -295,7 +308,10 @@ __global__ void __launch_bounds__(kPrepThreads, 4) prep_kernel(const DevPair *__
         const float pw[4] = S2_POW_TAB_INIT;
         lut[256 + threadIdx.x] = pw[threadIdx.x];
     }
-    for (int item = first_block + blockIdx.x; item < end_block; item += gridDim.x) {
+    const int items = (end_block - first_block) * (2 / kImgs);
+    for (int it = blockIdx.x; it < items; it += gridDim.x) {
+        const int item = first_block + (kImgs == 1 ? it >> 1 : it);
+        const int only = kImgs == 1 ? it & 1 : 0;
         int lo = 0, hi = npairs - 1;
         while (lo < hi) {
             int mid = (lo + hi + 1) >> 1;
@@ -307,24 +323,25 @@ __global__ void __launch_bounds__(kPrepThreads, 4) prep_kernel(const DevPair *__
             ((long long *)&sP)[i] = __ldg((const long long *)(pairs + lo) + i);
         __syncthreads();
         const DevPair &P = sP;
+        if (kImgs == 1 && !((P.prep_mask >> only) & 1)) continue;
         const int b = item - blk_first[lo];
         const int bx = b % P.blk_x, by = b / P.blk_x;
-        const int X0 = bx * kPyrBlk, Y0 = by * kPyrBlk;
+        const int X0 = bx * BLK, Y0 = by * BLK;
         if constexpr (FMT >= 0) {
-            prep_quads<(FMT >= 0 ? FMT : 0), ST, OUT>(P, X0, Y0, lut, cc, lv1);
+            prep_quads<(FMT >= 0 ? FMT : 0), ST, OUT, BLK>(P, X0, Y0, lut, cc, lv1, only);
         } else {
             switch (P.fmt) {
-            case FMT_LINEAR_F32: prep_quads<FMT_LINEAR_F32, ST, OUT>(P, X0, Y0, lut, cc, lv1); break;
-            case FMT_SRGB8: prep_quads<FMT_SRGB8, ST, OUT>(P, X0, Y0, lut, cc, lv1); break;
-            case FMT_NV12: prep_quads<FMT_NV12, ST, OUT>(P, X0, Y0, lut, cc, lv1); break;
-            case FMT_P016: prep_quads<FMT_P016, ST, OUT>(P, X0, Y0, lut, cc, lv1); break;
-            default: prep_quads<FMT_RGB16, ST, OUT>(P, X0, Y0, lut, cc, lv1); break;
+            case FMT_LINEAR_F32: prep_quads<FMT_LINEAR_F32, ST, OUT, BLK>(P, X0, Y0, lut, cc, lv1, only); break;
+            case FMT_SRGB8: prep_quads<FMT_SRGB8, ST, OUT, BLK>(P, X0, Y0, lut, cc, lv1, only); break;
+            case FMT_NV12: prep_quads<FMT_NV12, ST, OUT, BLK>(P, X0, Y0, lut, cc, lv1, only); break;
+            case FMT_P016: prep_quads<FMT_P016, ST, OUT, BLK>(P, X0, Y0, lut, cc, lv1, only); break;
+            default: prep_quads<FMT_RGB16, ST, OUT, BLK>(P, X0, Y0, lut, cc, lv1, only); break;
             }
         }
         __syncthreads();
         const int nlev = (OUT & 2) ? P.prep_levels : P.nscales;
         for (int s = 2; s < nlev; s++) {
-            const int bs = kPyrBlk >> s, pbs = kPyrBlk >> (s - 1);
+            const int bs = BLK >> s, pbs = BLK >> (s - 1);
             const int ox0 = X0 >> s, oy0 = Y0 >> s;
             const int px0 = X0 >> (s - 1), py0 = Y0 >> (s - 1);
             const int wp = P.w[s - 1], hp = P.h[s - 1];
@@ -336,16 +353,17 @@ __global__ void __launch_bounds__(kPrepThreads, 4) prep_kernel(const DevPair *__
                 const int ya = 2 * oy, yb = min(2 * oy + 1, hp - 1);
                 const int ia = (ya - py0) * pbs, ib = (yb - py0) * pbs;
                 const int ja = xa - px0, jb = xb - px0;
-                for (int img = 0; img < 2; img++) {
-                    if (!((P.prep_mask >> img) & 1)) continue;
+                for (int img = kImgs == 1 ? only : 0; img < (kImgs == 1 ? only + 1 : 2); img++) {
+                    if (kImgs == 2 && !((P.prep_mask >> img) & 1)) continue;
+                    const int at = kImgs == 1 ? 0 : img;
                     float v[3];
                     for (int c = 0; c < 3; c++) {
-                        const float *src = s == 2 ? lv1[img][c] : pp[(s - 1) & 1][img][c];
+                        const float *src = s == 2 ? lv1[at][c] : pp[(s - 1) & 1][at][c];
                         float sum = src[ia + ja] + src[ia + jb];
                         sum = sum + src[ib + ja];
                         sum = sum + src[ib + jb];
                         v[c] = sum * 0.25f;
-                        pp[s & 1][img][c][i] = v[c];
+                        pp[s & 1][at][c][i] = v[c];
                     }
                     if ((OUT & 1) && (!(OUT & 2) || s < P.nscales)) {
                         if (P.fmt == FMT_LINEAR_F32) store_xyb<ST, false>(P, img, s, ox, oy, v);
@@ -1037,44 +1055,49 @@ int fused_blocks_per_sm(int storage) {
 
 template <int OUT, int FMT>
 static void prep_launch_f(const DevPair *pairs, int npairs, const int *blk_first, int first_block, int end_block,
-                          const ColorConsts &cc, const float *lut, int grid, cudaStream_t st) {
-    prep_kernel<float, OUT, FMT>
-        <<<grid, kPrepThreads, 0, st>>>(pairs, npairs, blk_first, first_block, end_block, cc, lut);
+                          const ColorConsts &cc, const float *lut, int grid, cudaStream_t st, int edge) {
+    if (edge == kPyrBlkSmall)
+        prep_kernel<float, OUT, FMT, kPyrBlkSmall>
+            <<<grid, kPrepThreads, 0, st>>>(pairs, npairs, blk_first, first_block, end_block, cc, lut);
+    else
+        prep_kernel<float, OUT, FMT, kPyrBlk>
+            <<<grid, kPrepThreads, 0, st>>>(pairs, npairs, blk_first, first_block, end_block, cc, lut);
 }
 
 template <int OUT>
 static void prep_launch(const DevPair *pairs, int npairs, const int *blk_first, int first_block, int end_block,
-                        const ColorConsts &cc, const float *lut, int grid, cudaStream_t st, int fmt) {
+                        const ColorConsts &cc, const float *lut, int grid, cudaStream_t st, int fmt, int edge) {
     switch (fmt) {
     case FMT_LINEAR_F32:
-        prep_launch_f<OUT, FMT_LINEAR_F32>(pairs, npairs, blk_first, first_block, end_block, cc, lut, grid, st);
+        prep_launch_f<OUT, FMT_LINEAR_F32>(pairs, npairs, blk_first, first_block, end_block, cc, lut, grid, st, edge);
         break;
     case FMT_SRGB8:
-        prep_launch_f<OUT, FMT_SRGB8>(pairs, npairs, blk_first, first_block, end_block, cc, lut, grid, st);
+        prep_launch_f<OUT, FMT_SRGB8>(pairs, npairs, blk_first, first_block, end_block, cc, lut, grid, st, edge);
         break;
     case FMT_NV12:
-        prep_launch_f<OUT, FMT_NV12>(pairs, npairs, blk_first, first_block, end_block, cc, lut, grid, st);
+        prep_launch_f<OUT, FMT_NV12>(pairs, npairs, blk_first, first_block, end_block, cc, lut, grid, st, edge);
         break;
     case FMT_P016:
-        prep_launch_f<OUT, FMT_P016>(pairs, npairs, blk_first, first_block, end_block, cc, lut, grid, st);
+        prep_launch_f<OUT, FMT_P016>(pairs, npairs, blk_first, first_block, end_block, cc, lut, grid, st, edge);
         break;
     case FMT_RGB16:
-        prep_launch_f<OUT, FMT_RGB16>(pairs, npairs, blk_first, first_block, end_block, cc, lut, grid, st);
+        prep_launch_f<OUT, FMT_RGB16>(pairs, npairs, blk_first, first_block, end_block, cc, lut, grid, st, edge);
         break;
-    default: prep_launch_f<OUT, -1>(pairs, npairs, blk_first, first_block, end_block, cc, lut, grid, st); break;
+    default: prep_launch_f<OUT, -1>(pairs, npairs, blk_first, first_block, end_block, cc, lut, grid, st, edge); break;
     }
 }
 
 cudaError_t launch_pyramid(int storage, const DevPair *pairs, int npairs, const int *blk_first, int first_block,
                            int end_block, const ColorConsts &cc, const float *lut, int grid, cudaStream_t st,
-                           int out, int fmt) {
+                           int out, int fmt, int edge) {
     const int nb = end_block - first_block;
     if (nb <= 0) return cudaSuccess;
-    grid = grid > nb ? nb : grid;
+    const int items = edge == kPyrBlkSmall ? 2 * nb : nb;  // the small form takes a block's images apart
+    grid = grid > items ? items : grid;
     (void)storage;
-    if (out == 3) prep_launch<3>(pairs, npairs, blk_first, first_block, end_block, cc, lut, grid, st, fmt);
-    else if (out == 2) prep_launch<2>(pairs, npairs, blk_first, first_block, end_block, cc, lut, grid, st, fmt);
-    else prep_launch<1>(pairs, npairs, blk_first, first_block, end_block, cc, lut, grid, st, fmt);
+    if (out == 3) prep_launch<3>(pairs, npairs, blk_first, first_block, end_block, cc, lut, grid, st, fmt, edge);
+    else if (out == 2) prep_launch<2>(pairs, npairs, blk_first, first_block, end_block, cc, lut, grid, st, fmt, edge);
+    else prep_launch<1>(pairs, npairs, blk_first, first_block, end_block, cc, lut, grid, st, fmt, edge);
     return cudaGetLastError();
 }
 

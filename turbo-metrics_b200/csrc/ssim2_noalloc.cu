@@ -137,8 +137,8 @@ extern "C" s2_status s2_compute_srgb8_noalloc(const uint8_t *ref, size_t ref_pit
         P.w[s] = (P.w[s - 1] + 1) / 2;
         P.h[s] = (P.h[s - 1] + 1) / 2;
     }
-    P.blk_x = (P.w[0] + kPyrBlk - 1) / kPyrBlk;
-    P.blk_y = (P.h[0] + kPyrBlk - 1) / kPyrBlk;
+    P.blk_x = (P.w[0] + kPyrBlkSmall - 1) / kPyrBlkSmall;
+    P.blk_y = (P.h[0] + kPyrBlkSmall - 1) / kPyrBlkSmall;
     P.blk_base = 0;
     const int strip = kStripMid;
     Seg segs[kScales];
@@ -206,7 +206,8 @@ extern "C" s2_status s2_compute_srgb8_noalloc(const uint8_t *ref, size_t ref_pit
     int sms = 148, bps = fused_blocks_per_sm(ST_F32), dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (launch_pyramid(ST_F32, dp, 1, (const int *)(base + off_blk), 0, P.blk_x * P.blk_y, cc, lut, sms * 8, cs) !=
+    if (launch_pyramid(ST_F32, dp, 1, (const int *)(base + off_blk), 0, P.blk_x * P.blk_y, cc, lut, sms * 8, cs, 1, -1,
+                       kPyrBlkSmall) !=
             cudaSuccess ||
         launch_fused(ST_F32, dp, (const Seg *)(base + off_seg), nseg, 0, tiles, (int *)(base + kOffCounter),
                      tile_check((int *)(base + kOffCounter + 4)), (double *)(base + off_part), sms * bps,
