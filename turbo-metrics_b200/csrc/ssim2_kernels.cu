@@ -73,12 +73,17 @@ __device__ __forceinline__ void xyb3(const float l[3], float o[3]) {
     o[2] = xyb_from_opsin(2, a, b, c);
 }
 
-__device__ __forceinline__ int find_seg(const Seg *segs, int nseg, int tile) {
-    int lo = 0, hi = nseg - 1;
-    while (lo < hi) {
-        int mid = (lo + hi + 1) >> 1;
-        if (segs[mid].first_tile <= tile) lo = mid;
-        else hi = mid - 1;
+// The segment of a tile, by a whole warp: each round narrows the range 32
+// times (one round up to 32 segments, i.e. any single pair), where a binary
+// search waits for log2(nseg) loads one after the other.
+__device__ __forceinline__ int find_seg(const Seg *segs, int nseg, int tile, int lane) {
+    int lo = 0, n = nseg;  // the segment lies in [lo, lo + n)
+    while (n > 1) {
+        const int step = (n + 31) >> 5, i = lane * step;
+        const bool le = i < n && segs[lo + i].first_tile <= tile;
+        const int k = __popc(__ballot_sync(0xffffffffu, le)) - 1;
+        lo += k * step;
+        n = min(step, n - k * step);
     }
     return lo;
 }
@@ -782,11 +787,15 @@ __device__ __forceinline__ void issue_rows(const Item<ST> &it, int L, float *sta
 // load st + 3 right after the barrier that follows step st's vertical phase
 // (every thread has then read stage (st + 1) % 2, which it overwrites).  All
 // loads of an item are consumed before it ends.  `phase` holds each stage's
-// expected mbarrier parity (bit s), the same in every thread.
+// expected mbarrier parity (bit s), the same in every thread.  The block's next
+// item is claimed as the last step starts, so that the counter's answer is
+// there when the item ends; *s_next holds it (and *s_bad whether a wait ran
+// out) after the item's last barrier.
 template <typename ST, bool EXPORT>
-__device__ __forceinline__ bool flat_item(const Item<ST> &it, float2 *smb, float *stages, uint64_t *bars,
+__device__ __forceinline__ void flat_item(const Item<ST> &it, float2 *smb, float *stages, uint64_t *bars,
                                           unsigned &phase, const TileCheck &ck, int tid, double (*s_warp)[6],
-                                          double *__restrict__ partials, int item, const MapOut &mo) {
+                                          double *__restrict__ partials, int item, const MapOut &mo,
+                                          int *__restrict__ counter, int *s_next, int *s_bad) {
     const ItemGeo &G = it.G;
     const float cg = G.cg;
     const int x = G.x0 - 4 + tid;
@@ -820,9 +829,11 @@ __device__ __forceinline__ bool flat_item(const Item<ST> &it, float2 *smb, float
     double *sacc = (double *)(stages + kStages * kStageFloats) + tid;
 #pragma unroll
     for (int m = 0; m < 6; m++) sacc[m * kFusedThreads] = 0.0;
+    int next = 0;
     auto step = [&](int st, auto s0) {
         const int r = st * kStep, nr = min(kStep, it.rows_out - r);
         const int ybase = G.y0 + r + 4;
+        if (tid == 0 && st + 1 == it.nsteps) next = atomicAdd(counter, 1);
         wait(st + 1);
         StepRows in;
         v_load(in, stage(st + 1), tid, colin, ybase, G.H, cols_in && nr == kStep && ybase + kStep <= G.H, cg);
@@ -843,6 +854,8 @@ __device__ __forceinline__ bool flat_item(const Item<ST> &it, float2 *smb, float
         for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
         if ((tid & 31) == 0) s_warp[tid >> 5][m] = v;
     }
+    if (tid == 0) *s_next = next;
+    if (!ok) *s_bad = 1;
     __syncthreads();
     if (tid < 6) {
         double v = 0.0;
@@ -850,12 +863,14 @@ __device__ __forceinline__ bool flat_item(const Item<ST> &it, float2 *smb, float
         for (int w = 0; w < kFusedThreads / 32; w++) v += s_warp[w][tid];
         partials[(long long)item * 6 + tid] = v;  // = tile * 18 + channel * 6 + m
     }
-    return ok;
 }
 
-// Persistent: each block claims work items from the atomic counter until
-// they run out.  Dynamic shared memory: the step buffer, the two row stages,
-// the threads' f64 sums.  A block whose row copies time out (err set) stops claiming.
+// Persistent: block b starts with work item b and claims further ones from
+// the atomic counter until they run out (with the claim and a binary segment
+// search between two items, 64 x 1080p pairs took 2851 us instead of 2798).
+// Dynamic shared memory: the step
+// buffer, the two row stages, the threads' f64 sums.  A block whose row copies
+// time out (err set) stops claiming.
 template <typename ST, bool EXPORT = false>
 __global__ void __launch_bounds__(kFusedThreads, kTileBlocks)
     fused_kernel(const DevPair *__restrict__ pairs, const Seg *__restrict__ segs, int nseg, int first_item,
@@ -863,7 +878,7 @@ __global__ void __launch_bounds__(kFusedThreads, kTileBlocks)
                  MapOut mo = MapOut{nullptr, 0, 0}) {
     extern __shared__ __align__(128) float2 smb[];  // [3 planes][kStep][kRS], then the stages and sums
     float *const stages = (float *)(smb + kBufF2);
-    __shared__ int s_item, s_bad;
+    __shared__ int s_next, s_bad;
     __shared__ double s_warp[kFusedThreads / 32][6];
     __shared__ __align__(8) uint64_t s_bar[kStages];
     const int tid = threadIdx.x;
@@ -873,18 +888,16 @@ __global__ void __launch_bounds__(kFusedThreads, kTileBlocks)
         s_bad = 0;
         s2_wait_limit = ck.wait_cycles;
     }
+    __syncthreads();
     unsigned phase = 0;
-    for (;;) {
-        __syncthreads();  // the previous item's readers of s_item, s_warp and the buffers are done
-        if (tid == 0) s_item = s_bad ? end_item : first_item + atomicAdd(counter, 1);
-        __syncthreads();
-        const int item = s_item;
-        if (item >= end_item) break;
+    int item = first_item + blockIdx.x;  // the grid is at most the items
+    while (item < end_item) {
         const int tile = item / 3, g = item - 3 * tile;
-        const Seg sg = segs[find_seg(segs, nseg, tile)];
+        const Seg sg = segs[find_seg(segs, nseg, tile, tid & 31)];
         const Item<ST> it = decode_item<ST>(pairs[sg.pair], sg, tile, g);
-        if (!flat_item<ST, EXPORT>(it, smb, stages, s_bar, phase, ck, tid, s_warp, partials, item, mo))
-            s_bad = 1;
+        flat_item<ST, EXPORT>(it, smb, stages, s_bar, phase, ck, tid, s_warp, partials, item, mo, counter, &s_next,
+                              &s_bad);
+        item = s_bad ? end_item : first_item + (int)gridDim.x + s_next;
     }
     // after a time-out, give copies still in flight a bounded wait before the
     // block's shared memory goes away
