@@ -2,6 +2,8 @@
 import ctypes
 import os
 
+import numpy as np
+
 HERE = os.path.dirname(os.path.abspath(__file__))
 library_path = os.path.join(HERE, "libssim2b200.so")
 
@@ -95,6 +97,10 @@ class Result(ctypes.Structure):
                 ("dssim", ctypes.c_double), ("dssim_scale", ctypes.c_double * 5)]
 
 
+# the same structures as numpy types (arrays of them are filled and read in bulk)
+RESULT_DTYPE = np.dtype([("score", "f8"), ("stats", "f8", (NUM_STATS,)), ("sums", "f8", (NUM_STATS,)),
+                         ("n_scales", "i4"), ("status", "i4"), ("dssim", "f8"), ("dssim_scale", "f8", (5,))])
+
 METRIC = {"ssimulacra2": 1, "dssim": 2}
 
 
@@ -113,6 +119,12 @@ class PairDescC(ctypes.Structure):
                 ("bits", ctypes.c_int32), ("ref", ctypes.c_void_p), ("dis", ctypes.c_void_p),
                 ("ref_uv", ctypes.c_void_p), ("dis_uv", ctypes.c_void_p), ("ref_pitch", ctypes.c_size_t),
                 ("dis_pitch", ctypes.c_size_t), ("matrix", ctypes.c_int32), ("range", ctypes.c_int32)]
+
+
+PAIR_DTYPE = np.dtype([("width", "u4"), ("height", "u4"), ("format", "i4"), ("bits", "i4"), ("ref", "u8"),
+                       ("dis", "u8"), ("ref_uv", "u8"), ("dis_uv", "u8"), ("ref_pitch", "u8"), ("dis_pitch", "u8"),
+                       ("matrix", "i4"), ("range", "i4")])
+assert RESULT_DTYPE.itemsize == ctypes.sizeof(Result) and PAIR_DTYPE.itemsize == ctypes.sizeof(PairDescC)
 
 
 class ServerConfig(ctypes.Structure):
@@ -156,7 +168,7 @@ _sig = {
                                        ctypes.c_int32, ctypes.c_int32, P]),
     "s2_compute_rgb16": (ctypes.c_int, [P, P, ctypes.c_size_t, P, ctypes.c_size_t, ctypes.c_int32,
                                         ctypes.c_int32, P]),
-    "s2_get_result": (ctypes.c_int, [P, D, D, D]),
+    "s2_get_result": (ctypes.c_int, [P, P, P, P]),
     "s2_compute_sync_linear_f32": (ctypes.c_int, [P, P, ctypes.c_size_t, P, ctypes.c_size_t, P, D]),
     "s2_set_reference_linear_f32": (ctypes.c_int, [P, P, ctypes.c_size_t, P]),
     "s2_set_reference_srgb8": (ctypes.c_int, [P, P, ctypes.c_size_t, ctypes.c_int32, P]),

@@ -23,45 +23,53 @@ from . import capi
 from .capi import lib, check, NUM_STATS
 
 
+_torch = None  # torch, once it has found a CUDA device
+
+
 def _stream_ptr(stream):
+    global _torch
     if stream is None:
-        try:
-            import torch
-            if torch.cuda.is_available():
-                return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-        except ImportError:
-            pass
-        return None
+        if _torch is None:
+            try:
+                import torch
+            except ImportError:
+                return None
+            if not torch.cuda.is_available():
+                return None
+            _torch = torch
+        return _torch.cuda.current_stream().cuda_stream
     if isinstance(stream, int):
-        return ctypes.c_void_p(stream)
-    return ctypes.c_void_p(stream.cuda_stream)
+        return stream
+    return stream.cuda_stream
 
 
 def _dev(img, elem_bytes):
-    """(pointer, pitch in bytes) of a device image."""
+    """(address, pitch in bytes) of a device image."""
     if isinstance(img, tuple):
-        return ctypes.c_void_p(img[0]), img[1]
+        return img[0], img[1]
     if not img.is_cuda:
         raise capi.S2Error(capi.S2_ERR_INVALID_ARG, "expected a CUDA tensor")
-    if img.stride(-1) != 1 or (img.dim() == 3 and img.stride(1) != img.shape[2]):
+    stride = img.stride()
+    if stride[-1] != 1 or (len(stride) == 3 and stride[1] != img.shape[2]):
         raise capi.S2Error(capi.S2_ERR_INVALID_ARG, "rows must be packed samples")
-    return ctypes.c_void_p(img.data_ptr()), img.stride(0) * elem_bytes
+    return img.data_ptr(), stride[0] * elem_bytes
 
 
 def _host_ptr(img, elem_bytes):
-    """(pointer, pitch in bytes) of a host image: a CPU torch tensor (pinned
+    """(address, pitch in bytes) of a host image: a CPU torch tensor (pinned
     for asynchronous uploads) or a numpy array with packed rows."""
     if isinstance(img, tuple):
-        return ctypes.c_void_p(img[0]), img[1]
+        return img[0], img[1]
     if isinstance(img, np.ndarray):
         if img.strides[-1] != img.itemsize or (img.ndim == 3 and img.strides[1] != img.shape[2] * img.itemsize):
             raise capi.S2Error(capi.S2_ERR_INVALID_ARG, "rows must be packed samples")
-        return ctypes.c_void_p(img.ctypes.data), img.strides[0]
+        return img.ctypes.data, img.strides[0]
     if img.is_cuda:
         raise capi.S2Error(capi.S2_ERR_INVALID_ARG, "expected a host (CPU) tensor")
-    if img.stride(-1) != 1 or (img.dim() == 3 and img.stride(1) != img.shape[2]):
+    stride = img.stride()
+    if stride[-1] != 1 or (len(stride) == 3 and stride[1] != img.shape[2]):
         raise capi.S2Error(capi.S2_ERR_INVALID_ARG, "rows must be packed samples")
-    return ctypes.c_void_p(img.data_ptr()), img.stride(0) * elem_bytes
+    return img.data_ptr(), stride[0] * elem_bytes
 
 
 def _host(img):
@@ -161,12 +169,11 @@ class Ssimulacra2:
 
     def get_result(self):
         """(score, stats[108], sums[108]) of the last compute."""
+        out = np.empty((2, NUM_STATS))
         sc = ctypes.c_double()
-        st = np.zeros(NUM_STATS)
-        su = np.zeros(NUM_STATS)
-        check(lib.s2_get_result(self._h, ctypes.byref(sc), st.ctypes.data_as(capi.D),
-                                su.ctypes.data_as(capi.D)), "get_score")
-        return sc.value, st, su
+        at = out.ctypes.data
+        check(lib.s2_get_result(self._h, ctypes.byref(sc), at, at + 8 * NUM_STATS), "get_score")
+        return sc.value, out[0], out[1]
 
     def compute_linear(self, ref, dis, stream=None):
         rp, rpitch = _dev(ref, 4)
@@ -277,6 +284,9 @@ class Ssimulacra2:
             raise capi.DimensionMismatch(capi.S2_ERR_DIM_MISMATCH, "host image shape")
 
 
+_ELEM_BYTES = {"linear_f32": 4, "srgb8": 1, "nv12": 1, "rgb16": 2, "p016": 2}
+
+
 class PairDesc:
     """One pair of a batch: device tensors of any supported format (host arrays
     for `Ssim2Batch.submit_host`)."""
@@ -285,23 +295,36 @@ class PairDesc:
         self.ref, self.dis, self.fmt, self.ref_uv, self.dis_uv, self.bits = ref, dis, fmt, ref_uv, dis_uv, bits
         self.matrix, self.range = matrix, range
 
-    def to_c(self, host=False):
-        d = capi.PairDescC()
-        eb = {"linear_f32": 4, "srgb8": 1, "nv12": 1, "rgb16": 2, "p016": 2}[self.fmt]
+    def _row(self, host=False, dis_only=False):
+        """The pair's fields in the order of capi.PAIR_DTYPE (dis_only: a
+        candidate of a cached reference)."""
+        eb = _ELEM_BYTES[self.fmt]
         ptr = _host_ptr if host else _dev
         rp, rpitch = ptr(self.ref, eb)
-        dp, dpitch = ptr(self.dis, eb)
-        d.height, d.width = self.ref.shape[0], self.ref.shape[1]
-        d.format = capi.FMT[self.fmt]
-        d.bits = self.bits
-        d.ref, d.dis = rp.value, dp.value
-        d.ref_pitch, d.dis_pitch = rpitch, dpitch
+        dp, dpitch = (rp, rpitch) if self.dis is self.ref else ptr(self.dis, eb)
+        shape = self.ref.shape
+        ru = du = matrix = range_ = 0
         if self.fmt in ("nv12", "p016"):
-            d.ref_uv = ptr(self.ref_uv, eb)[0].value
-            d.dis_uv = ptr(self.dis_uv, eb)[0].value
-            d.matrix = capi.MATRIX[self.matrix]
-            d.range = capi.RANGE[self.range]
+            ru = ptr(self.ref_uv, eb)[0]
+            du = ru if self.dis_uv is self.ref_uv else ptr(self.dis_uv, eb)[0]
+            matrix, range_ = capi.MATRIX[self.matrix], capi.RANGE[self.range]
+        if dis_only:
+            rp = ru = 0
+        return (shape[1], shape[0], capi.FMT[self.fmt], self.bits, rp, dp, ru, du, rpitch, dpitch, matrix, range_)
+
+    def to_c(self, host=False):
+        d = capi.PairDescC()
+        (d.width, d.height, d.format, d.bits, d.ref, d.dis, ru, du, d.ref_pitch, d.dis_pitch, d.matrix,
+         d.range) = self._row(host)
+        if self.fmt in ("nv12", "p016"):
+            d.ref_uv, d.dis_uv = ru, du
         return d
+
+
+def _descs(rows):
+    """The C descriptors of a submission: (array that owns them, pointer)."""
+    a = np.array(rows, dtype=capi.PAIR_DTYPE) if rows else np.zeros(1, dtype=capi.PAIR_DTYPE)
+    return a, ctypes.cast(a.ctypes.data, ctypes.POINTER(capi.PairDescC))
 
 
 class Ssim2Batch:
@@ -340,9 +363,7 @@ class Ssim2Batch:
         self.close()
 
     def submit(self, pairs, stream=None):
-        arr = (capi.PairDescC * max(len(pairs), 1))()
-        for i, p in enumerate(pairs):
-            arr[i] = p.to_c()
+        keep, arr = _descs([p._row() for p in pairs])
         k = self._take_slot(False)
         check(lib.s2_batch_submit(self._h, arr, len(pairs), _stream_ptr(stream)), "compute_batch")
         self._last = (k, len(pairs), pairs)
@@ -365,9 +386,7 @@ class Ssim2Batch:
         `results()` returns.  A second host submission may be made before
         reading the first one's results: its uploads and preps then overlap
         the first one's tile pass (results are read oldest first)."""
-        arr = (capi.PairDescC * max(len(pairs), 1))()
-        for i, p in enumerate(pairs):
-            arr[i] = p.to_c(host=True)
+        keep, arr = _descs([p._row(True) for p in pairs])
         k = self._take_slot(True)
         check(lib.s2_batch_submit_host(self._h, arr, len(pairs), _stream_ptr(stream)), "compute_batch_host")
         self._last = (k, len(pairs), pairs)
@@ -376,10 +395,12 @@ class Ssim2Batch:
     def results(self):
         """Results of the oldest submission not read yet (else the last one)."""
         _, n, _ = self._unread.popleft() if self._unread else self._last
-        out = (capi.Result * max(n, 1))()
-        check(lib.s2_batch_results(self._h, out, n), "results")
-        return [(r.score, np.array(r.stats[:]), np.array(r.sums[:]), r.n_scales, r.status, r.dssim,
-                 np.array(r.dssim_scale[:])) for r in out[:n]]
+        out = np.empty(max(n, 1), dtype=capi.RESULT_DTYPE)
+        check(lib.s2_batch_results(self._h, ctypes.cast(out.ctypes.data, ctypes.POINTER(capi.Result)), n), "results")
+        out = out[:n]
+        # each field in an array of its own, whose rows the tuples hold
+        return list(zip(out["score"].tolist(), out["stats"].copy(), out["sums"].copy(), out["n_scales"].tolist(),
+                        out["status"].tolist(), out["dssim"].tolist(), out["dssim_scale"].copy()))
 
     def compute_batch(self, pairs, stream=None):
         self.submit(pairs, stream)
@@ -402,10 +423,11 @@ class Ssim2Batch:
     def submit_with_reference(self, dis, fmt="srgb8", dis_uv=None, stream=None, **kw):
         """Enqueue distorted images (device tensors, one size) against the
         cached reference; `dis_uv` gives their CbCr planes for 4:2:0 input."""
-        arr = (capi.PairDescC * max(len(dis), 1))()
+        rows = []
         for i, t in enumerate(dis):
-            arr[i] = PairDesc(t, t, fmt, dis_uv[i] if dis_uv else None, dis_uv[i] if dis_uv else None, **kw).to_c()
-            arr[i].ref = arr[i].ref_uv = None
+            uv = dis_uv[i] if dis_uv else None
+            rows.append(PairDesc(t, t, fmt, uv, uv, **kw)._row(dis_only=True))
+        keep, arr = _descs(rows)
         k = self._take_slot(False)
         check(lib.s2_batch_submit_with_reference(self._h, arr, len(dis), _stream_ptr(stream)), "compute_batch")
         self._last = (k, len(dis), (dis, dis_uv))
