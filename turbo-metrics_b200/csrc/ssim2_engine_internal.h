@@ -188,7 +188,12 @@ struct Engine {
     DevBuf pairs_d, blk_d, segs_d, counter_d, partials_d, results_d, levels_d, lut_d, iir_d;
     // counter_d: the tile groups' work counters (ints 0..), and at its last
     // int the tile pass's error word; all zeroed before every submission
-    static constexpr size_t kCounterBytes = 256;
+    static constexpr size_t kCounterBytes = kCounterInts * sizeof(int);
+    // Where a submission's results are formed: for a few pairs the page-locked
+    // host array itself (the last kernels' stores cross the link, 1.8 KB a
+    // pair), which saves the copy behind them; else device memory and one copy.
+    static constexpr int kDirectPairs = 4;
+    DevResult *results_at(int n) const { return n <= kDirectPairs ? results_h : (DevResult *)results_d.p; }
     int *err_word() const { return (int *)counter_d.p + kCounterBytes / sizeof(int) - 1; }
     DevBuf ds_d;  // DSSIM: per-tile SSIM sums, per-tile |avg - ssim| sums, per-level avg
     void *pinned = nullptr;  // staging: pairs | blk_first | segs
@@ -814,7 +819,10 @@ struct Engine {
             S2_CUDA(cudaEventRecord(sub_start, copy_st));
             S2_CUDA(cudaStreamWaitEvent(st, sub_start, 0));
         }
-        S2_CUDA(cudaMemsetAsync(counter_d.p, 0, kCounterBytes, st));
+        // the prep pass zeroes the counters, unless its groups run beside the tile
+        // passes or no pair has a block
+        const bool zero = !split && P.total_blocks > 0;
+        if (!zero) S2_CUDA(cudaMemsetAsync(counter_d.p, 0, kCounterBytes, st));
         if (profiling) S2_CUDA(cudaEventRecord(prof[0], st));
         cudaStream_t pst = split ? prep_st : st;
         for (int g = 0; g < ng; g++) {
@@ -842,7 +850,7 @@ struct Engine {
             const int b0 = pa < n ? P.blk_first[pa] : P.total_blocks;
             const int b1 = pe < n ? P.blk_first[pe] : P.total_blocks;
             S2_CUDA(launch_pyramid(storage, dpairs, n, dblk, b0, b1, cc, (const float *)lut_d.p, num_sms * 8, pst,
-                                   pout, uniform_fmt(P), P.pyr_blk));
+                                   pout, uniform_fmt(P), P.pyr_blk, zero ? (int *)counter_d.p : nullptr));
             if (host && g + 1 == ng) S2_CUDA(cudaEventRecord(stage_free, pst));
             if (split) {
                 S2_CUDA(cudaEventRecord(grp_prepped[g], prep_st));
@@ -857,17 +865,19 @@ struct Engine {
             else
                 S2_CUDA(launch_fused(storage, dpairs, dsegs, (int)P.segs.size(), P.grp_tile[g], P.grp_tile[g + 1],
                                      (int *)counter_d.p + g, tile_check(err_word()), (double *)partials_d.p, num_sms * fused_bps,
-                                     st));
+                                     st, !split));
         }
         // several groups interleave prep and fused: the fused slot then holds both
         if (profiling && ng > 1) S2_CUDA(cudaEventRecord(prof[1], st));
         if (profiling) S2_CUDA(cudaEventRecord(prof[2], st));
         if (m_s2)
-            S2_CUDA(launch_finalize(dpairs, n, (const double *)partials_d.p, err_word(), (DevResult *)results_d.p, st));
+            S2_CUDA(launch_finalize(dpairs, n, (const double *)partials_d.p, err_word(), results_at(n), st,
+                                    !split && blur != S2_BLUR_IIR_REF));
         if (profiling) S2_CUDA(cudaEventRecord(prof[3], st));
         if (m_ds) S2_CUDA(launch_ds(P, dbase, st));
         if (profiling) S2_CUDA(cudaEventRecord(prof[4], st));
-        S2_CUDA(cudaMemcpyAsync(results_h, results_d.p, n * sizeof(DevResult), cudaMemcpyDeviceToHost, st));
+        if (results_at(n) != results_h)
+            S2_CUDA(cudaMemcpyAsync(results_h, results_d.p, n * sizeof(DevResult), cudaMemcpyDeviceToHost, st));
         S2_CUDA(cudaEventRecord(done, st));
         last_n = n;
         pending = true;
@@ -886,7 +896,7 @@ struct Engine {
         double *part = (double *)ds_d.p;
         float *avg = (float *)((char *)ds_d.p + s2_align_up((size_t)2 * std::max(P.ds_tiles, 1) * sizeof(double), 256));
         return launch_dssim((const DsPair *)(dbase + L.ds_pairs()), n, (const DsSeg *)(dbase + L.ds_segs()),
-                            (int)P.dsegs.size(), P.ds_tiles, P.ds_clamp, part, avg, (DevResult *)results_d.p,
+                            (int)P.dsegs.size(), P.ds_tiles, P.ds_clamp, part, avg, results_at(n),
                             (P.metrics & S2_METRIC_SSIMULACRA2) == 0, num_sms, st);
     }
 
@@ -912,11 +922,12 @@ struct Engine {
         }
         cudaError_t e = desc_kernel ? launch_desc_copy(dbase, pinned_dev, desc_bytes, cap_st)
                                     : cudaMemcpyAsync(dbase, pinned, desc_bytes, cudaMemcpyHostToDevice, cap_st);
-        if (e == cudaSuccess) e = cudaMemsetAsync(counter_d.p, 0, kCounterBytes, cap_st);
+        const bool zero = P.total_blocks > 0;
+        if (e == cudaSuccess && !zero) e = cudaMemsetAsync(counter_d.p, 0, kCounterBytes, cap_st);
         if (e == cudaSuccess)
             e = launch_pyramid(storage, dpairs, n, (const int *)(dbase + pb), 0, P.total_blocks, cc,
                                (const float *)lut_d.p, num_sms * 8, cap_st, (m_s2 ? 1 : 0) | (m_ds ? 2 : 0),
-                               uniform_fmt(P), P.pyr_blk);
+                               uniform_fmt(P), P.pyr_blk, zero ? (int *)counter_d.p : nullptr);
         if (e == cudaSuccess && m_s2) {
             if (blur == S2_BLUR_IIR_REF)
                 e = launch_iir(storage, dpairs, (const IirSeg *)(dbase + pb + bb + sb), (int)P.vsegs.size(), P.vtotal,
@@ -925,12 +936,13 @@ struct Engine {
             else
                 e = launch_fused(storage, dpairs, (const Seg *)(dbase + pb + bb), (int)P.segs.size(), 0,
                                  P.total_tiles, (int *)counter_d.p, tile_check(err_word()), (double *)partials_d.p,
-                                 num_sms * fused_bps, cap_st);
+                                 num_sms * fused_bps, cap_st, true);
         }
         if (e == cudaSuccess && m_s2)
-            e = launch_finalize(dpairs, n, (const double *)partials_d.p, err_word(), (DevResult *)results_d.p, cap_st);
+            e = launch_finalize(dpairs, n, (const double *)partials_d.p, err_word(), results_at(n), cap_st,
+                                blur != S2_BLUR_IIR_REF);
         if (e == cudaSuccess && m_ds) e = launch_ds(P, dbase, cap_st);
-        if (e == cudaSuccess)
+        if (e == cudaSuccess && results_at(n) != results_h)
             e = cudaMemcpyAsync(results_h, results_d.p, n * sizeof(DevResult), cudaMemcpyDeviceToHost, cap_st);
         cudaGraph_t graph = nullptr;
         const cudaError_t ee = cudaStreamEndCapture(cap_st, &graph);

@@ -33,6 +33,15 @@
 
 namespace s2 {
 
+// Programmatic dependent launch: a kernel launched with it starts as soon as
+// the blocks of the one before it in the stream have all started (they say so
+// first thing), sets itself up, and waits here until that one is complete.
+// With the counters zeroed by the prep pass and a few pairs' results stored
+// straight to host memory, a 96x64 pair's call went from 47.3 to 34.4 us and a
+// 1920x1080 one's from 131 to 119 (three graph nodes and two launch latencies).
+__device__ __forceinline__ void s2_grid_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void s2_grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Shared memory of fused_kernel (one CTA = one channel of a tile): the step
 // buffer, three float2 planes of kStep rows x kRS columns -- plane 0 and 1
 // the vertical FIRs, plane 2 the raw (x', e) of the output rows -- then two
@@ -298,7 +307,11 @@ template <typename ST, int OUT, int FMT, int BLK>
 __global__ void __launch_bounds__(kPrepThreads, 4) prep_kernel(const DevPair *__restrict__ pairs, int npairs,
                                                    const int *__restrict__ blk_first, int first_block,
                                                    int end_block,
-                                                   ColorConsts cc, const float *__restrict__ lut_g) {
+                                                   ColorConsts cc, const float *__restrict__ lut_g,
+                                                   int *__restrict__ zero) {
+    s2_grid_start();
+    // the tile pass's work counters and time-out word, for the pass that follows
+    if (zero && blockIdx.x == 0 && threadIdx.x < kCounterInts) zero[threadIdx.x] = 0;
     constexpr int kLv1 = BLK / 2;
     constexpr int kImgs = BLK == kPyrBlkSmall ? 1 : 2;        // images of a block
     __shared__ float lv1[kImgs][3][kLv1 * kLv1];              // scale-1 linear block [img][ch][px]
@@ -888,6 +901,8 @@ __global__ void __launch_bounds__(kFusedThreads, kTileBlocks)
         s_bad = 0;
         s2_wait_limit = ck.wait_cycles;
     }
+    s2_grid_start();
+    s2_grid_wait();  // the planes are written
     __syncthreads();
     unsigned phase = 0;
     int item = first_item + blockIdx.x;  // the grid is at most the items
@@ -932,6 +947,7 @@ __global__ void __launch_bounds__(kFinThreads) finalize_kernel(const DevPair *__
                                                                DevResult *__restrict__ out) {
     __shared__ double red[kFinGroups][108];
     __shared__ double st[108];
+    s2_grid_wait();  // the tile records are written
     const int p = blockIdx.x;
     const DevPair &P = pairs[p];
     const int t = threadIdx.x, g = t / 18, j = t % 18;
@@ -1068,62 +1084,79 @@ int fused_blocks_per_sm(int storage) {
 
 template <int OUT, int FMT>
 static void prep_launch_f(const DevPair *pairs, int npairs, const int *blk_first, int first_block, int end_block,
-                          const ColorConsts &cc, const float *lut, int grid, cudaStream_t st, int edge) {
+                          const ColorConsts &cc, const float *lut, int grid, cudaStream_t st, int edge, int *zero) {
     if (edge == kPyrBlkSmall)
         prep_kernel<float, OUT, FMT, kPyrBlkSmall>
-            <<<grid, kPrepThreads, 0, st>>>(pairs, npairs, blk_first, first_block, end_block, cc, lut);
+            <<<grid, kPrepThreads, 0, st>>>(pairs, npairs, blk_first, first_block, end_block, cc, lut, zero);
     else
         prep_kernel<float, OUT, FMT, kPyrBlk>
-            <<<grid, kPrepThreads, 0, st>>>(pairs, npairs, blk_first, first_block, end_block, cc, lut);
+            <<<grid, kPrepThreads, 0, st>>>(pairs, npairs, blk_first, first_block, end_block, cc, lut, zero);
 }
 
 template <int OUT>
 static void prep_launch(const DevPair *pairs, int npairs, const int *blk_first, int first_block, int end_block,
-                        const ColorConsts &cc, const float *lut, int grid, cudaStream_t st, int fmt, int edge) {
+                        const ColorConsts &cc, const float *lut, int grid, cudaStream_t st, int fmt, int edge,
+                        int *zero) {
     switch (fmt) {
     case FMT_LINEAR_F32:
-        prep_launch_f<OUT, FMT_LINEAR_F32>(pairs, npairs, blk_first, first_block, end_block, cc, lut, grid, st, edge);
+        prep_launch_f<OUT, FMT_LINEAR_F32>(pairs, npairs, blk_first, first_block, end_block, cc, lut, grid, st, edge, zero);
         break;
     case FMT_SRGB8:
-        prep_launch_f<OUT, FMT_SRGB8>(pairs, npairs, blk_first, first_block, end_block, cc, lut, grid, st, edge);
+        prep_launch_f<OUT, FMT_SRGB8>(pairs, npairs, blk_first, first_block, end_block, cc, lut, grid, st, edge, zero);
         break;
     case FMT_NV12:
-        prep_launch_f<OUT, FMT_NV12>(pairs, npairs, blk_first, first_block, end_block, cc, lut, grid, st, edge);
+        prep_launch_f<OUT, FMT_NV12>(pairs, npairs, blk_first, first_block, end_block, cc, lut, grid, st, edge, zero);
         break;
     case FMT_P016:
-        prep_launch_f<OUT, FMT_P016>(pairs, npairs, blk_first, first_block, end_block, cc, lut, grid, st, edge);
+        prep_launch_f<OUT, FMT_P016>(pairs, npairs, blk_first, first_block, end_block, cc, lut, grid, st, edge, zero);
         break;
     case FMT_RGB16:
-        prep_launch_f<OUT, FMT_RGB16>(pairs, npairs, blk_first, first_block, end_block, cc, lut, grid, st, edge);
+        prep_launch_f<OUT, FMT_RGB16>(pairs, npairs, blk_first, first_block, end_block, cc, lut, grid, st, edge, zero);
         break;
-    default: prep_launch_f<OUT, -1>(pairs, npairs, blk_first, first_block, end_block, cc, lut, grid, st, edge); break;
+    default: prep_launch_f<OUT, -1>(pairs, npairs, blk_first, first_block, end_block, cc, lut, grid, st, edge, zero); break;
     }
 }
 
 cudaError_t launch_pyramid(int storage, const DevPair *pairs, int npairs, const int *blk_first, int first_block,
                            int end_block, const ColorConsts &cc, const float *lut, int grid, cudaStream_t st,
-                           int out, int fmt, int edge) {
+                           int out, int fmt, int edge, int *zero) {
     const int nb = end_block - first_block;
     if (nb <= 0) return cudaSuccess;
     const int items = edge == kPyrBlkSmall ? 2 * nb : nb;  // the small form takes a block's images apart
     grid = grid > items ? items : grid;
     (void)storage;
-    if (out == 3) prep_launch<3>(pairs, npairs, blk_first, first_block, end_block, cc, lut, grid, st, fmt, edge);
-    else if (out == 2) prep_launch<2>(pairs, npairs, blk_first, first_block, end_block, cc, lut, grid, st, fmt, edge);
-    else prep_launch<1>(pairs, npairs, blk_first, first_block, end_block, cc, lut, grid, st, fmt, edge);
+    if (out == 3) prep_launch<3>(pairs, npairs, blk_first, first_block, end_block, cc, lut, grid, st, fmt, edge, zero);
+    else if (out == 2) prep_launch<2>(pairs, npairs, blk_first, first_block, end_block, cc, lut, grid, st, fmt, edge, zero);
+    else prep_launch<1>(pairs, npairs, blk_first, first_block, end_block, cc, lut, grid, st, fmt, edge, zero);
     return cudaGetLastError();
 }
 
+// Launch with or without programmatic dependence on the kernel before it.
+template <typename... Params, typename... Args>
+static cudaError_t launch_after(bool early, void (*kernel)(Params...), int grid, int block, size_t smem, cudaStream_t st,
+                                Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = early ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
+}
+
 cudaError_t launch_fused(int storage, const DevPair *pairs, const Seg *segs, int nseg, int first_tile, int end_tile,
-                         int *counter, const TileCheck &ck, double *partials, int grid, cudaStream_t st) {
+                         int *counter, const TileCheck &ck, double *partials, int grid, cudaStream_t st, bool early) {
     const int fi = 3 * first_tile, ei = 3 * end_tile;  // work items: (tile, channel)
     const int nt = ei - fi;
     if (nt <= 0) return cudaSuccess;
     grid = grid > nt ? nt : grid;
     (void)storage;
-    fused_kernel<float, false><<<grid, kTileThreads, fused_smem_bytes(), st>>>(pairs, segs, nseg, fi, ei, counter,
-                                                                              ck, partials, MapOut{nullptr, 0, 0});
-    return cudaGetLastError();
+    return launch_after(early, fused_kernel<float, false>, grid, kTileThreads, fused_smem_bytes(), st, pairs, segs, nseg,
+                        fi, ei, counter, ck, partials, MapOut{nullptr, 0, 0});
 }
 
 cudaError_t launch_fused_export(int storage, const DevPair *pairs, const Seg *segs, int nseg, int first_tile,
@@ -1154,10 +1187,9 @@ cudaError_t launch_desc_copy(void *dst, const void *src_host_mapped, size_t byte
 }
 
 cudaError_t launch_finalize(const DevPair *pairs, int npairs, const double *partials, const int *err,
-                            DevResult *out, cudaStream_t st) {
+                            DevResult *out, cudaStream_t st, bool early) {
     if (npairs <= 0) return cudaSuccess;
-    finalize_kernel<<<npairs, kFinThreads, 0, st>>>(pairs, npairs, partials, err, out);
-    return cudaGetLastError();
+    return launch_after(early, finalize_kernel, npairs, kFinThreads, 0, st, pairs, npairs, partials, err, out);
 }
 
 }  // namespace s2

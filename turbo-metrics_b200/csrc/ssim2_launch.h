@@ -16,9 +16,12 @@ int fused_blocks_per_sm(int storage);
 // (DSSIM), 3 both from one pass.  fmt: the input format shared by every
 // pair of the launch (a kernel compiled for it), or -1 for a mix.  edge: the
 // block edge that the blocks were counted with (kPyrBlk or kPyrBlkSmall).
+// zero: kCounterInts ints that the pass zeroes (the counters and the time-out
+// word of a tile pass that follows it), or nullptr.
+constexpr int kCounterInts = 64;
 cudaError_t launch_pyramid(int storage, const DevPair *pairs, int npairs, const int *blk_first, int first_block,
                            int end_block, const ColorConsts &cc, const float *lut, int grid, cudaStream_t st,
-                           int out = 1, int fmt = -1, int edge = kPyrBlk);
+                           int out = 1, int fmt = -1, int edge = kPyrBlk, int *zero = nullptr);
 // The tile pass's bounded waits: err is a device word (zeroed before the
 // submission) that a pass whose row copies time out sets (launch_finalize
 // then marks every pair S2_ERR_TIMEOUT); wait_cycles bounds each wait (SM
@@ -29,10 +32,13 @@ struct TileCheck {
     long long wait_cycles;
     int drop_item;
 };
+// early (launch_fused, launch_finalize): programmatic dependent launch after
+// the kernel before it in the stream -- the prep and the tile pass of the same
+// submission -- which hides the launch's latency.
 TileCheck tile_check(int *err);  // the process-wide setting (s2_debug_tile_timeout)
 cudaError_t launch_fused(int storage, const DevPair *pairs, const Seg *segs, int nseg, int first_tile,
                          int end_tile, int *counter, const TileCheck &ck, double *partials, int grid,
-                         cudaStream_t st);
+                         cudaStream_t st, bool early = false);
 // vtotal, htotal: blocks of the vertical and the horizontal walk
 cudaError_t configure_iir_kernels();
 cudaError_t launch_iir(int storage, const DevPair *pairs, const IirSeg *vsegs, int nvseg, int vtotal,
@@ -50,7 +56,7 @@ cudaError_t launch_fused_export(int storage, const DevPair *pairs, const Seg *se
                                 float *maps,
                                 long long mpitch, long long mplane, int grid, cudaStream_t st);
 cudaError_t launch_finalize(const DevPair *pairs, int npairs, const double *partials, const int *err,
-                            DevResult *out, cudaStream_t st);
+                            DevResult *out, cudaStream_t st, bool early = false);
 
 // DSSIM over the Lab planes of a submission (dssim_kernels.cu): the clamp
 // pass (levels clamped to 8 pixels, pairs with clamp_from < 5), the tile
