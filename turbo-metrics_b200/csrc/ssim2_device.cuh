@@ -253,61 +253,6 @@ __device__ __forceinline__ float s2_div(float a, float b) {
     return fmaf(e, r, q);
 }
 
-// 2^(r/9), r = 0..8, rounded to f32
-__device__ __forceinline__ float s2_pow2_r9(int r) {
-    const float lo = r < 2 ? (r == 0 ? 0x1p+0f : 0x1.147eccp+0f) : (r == 2 ? 0x1.2aa1a6p+0f : 0x1.428a3p+0f);
-    const float mid = r < 6 ? (r == 4 ? 0x1.5c5cbcp+0f : 0x1.784086p+0f) : (r == 6 ? 0x1.965feap+0f : 0x1.b6e8aep+0f);
-    return r < 4 ? lo : (r < 8 ? mid : 0x1.da0c4p+0f);
-}
-
-// p^(20/9) for normal p > 0 (the BT.709 inverse OETF exponent 1/0.45 =
-// 20/9), 0 for p <= 0.  With p = m 2^e, m in [1, 2): m^(20/9) is a degree-7
-// polynomial in t = m - 1.5 (Chebyshev interpolation at 8 nodes, converted
-// to monomials and rounded to f32; Horner with fmaf), times 2^(20e/9) =
-// 2^(2e + k) 2^(r/9) with 2e = 9k + r, 0 <= r < 9.  Branch-free; <= 3.3 ulp
-// on [0.1, 2].
-__device__ __forceinline__ float s2_pow_20_9(float p) {
-    const bool pos = p > 0.0f;
-    const unsigned b = __float_as_uint(pos ? p : 1.0f);
-    const int e = (int)((b >> 23) & 0xffu) - 127;
-    const float t = __uint_as_float((b & 0x7fffffu) | 0x3f800000u) - 1.5f;
-    float y = 0x1.1eb37ap-12f;
-    y = fmaf(y, t, -0x1.88e318p-11f);
-    y = fmaf(y, t, 0x1.2713a6p-9f);
-    y = fmaf(y, t, -0x1.37717ep-7f);
-    y = fmaf(y, t, 0x1.2c9724p-4f);
-    y = fmaf(y, t, 0x1.7c6f02p+0f);
-    y = fmaf(y, t, 0x1.d2e55cp+1f);
-    y = fmaf(y, t, 0x1.3b279ep+1f);
-    const int n = 2 * e;
-    const int k = (n + 261) / 9 - 29;  // floor(n / 9) for n >= -261
-    const int r = n - 9 * k;
-    y = y * s2_pow2_r9(r);
-    y = y * __uint_as_float((unsigned)(2 * e + k + 127) << 23);
-    return pos ? y : 0.0f;
-}
-
-// s2_pow_20_9 for p in [1/8, 2): there the exponent e is -3..0 and the
-// product of 2^(r/9) and 2^(2e + k) is one f32 constant 2^(20e/9) (a power
-// of two times the rounded 2^(r/9), so multiplying by it rounds exactly as
-// the two multiplications do): the same result from 4 selects instead of
-// the exponent arithmetic.
-__device__ __forceinline__ float s2_pow_20_9_unit(float p) {
-    const unsigned b = __float_as_uint(p);
-    const int e = (int)(b >> 23) - 127;
-    const float t = __uint_as_float((b & 0x7fffffu) | 0x3f800000u) - 1.5f;
-    float y = 0x1.1eb37ap-12f;
-    y = fmaf(y, t, -0x1.88e318p-11f);
-    y = fmaf(y, t, 0x1.2713a6p-9f);
-    y = fmaf(y, t, -0x1.37717ep-7f);
-    y = fmaf(y, t, 0x1.2c9724p-4f);
-    y = fmaf(y, t, 0x1.7c6f02p+0f);
-    y = fmaf(y, t, 0x1.d2e55cp+1f);
-    y = fmaf(y, t, 0x1.3b279ep+1f);
-    const float s = e == 0 ? 1.0f : (e == -1 ? 0x1.b6e8aep-3f : (e == -2 ? 0x1.784086p-5f : 0x1.428a3p-7f));
-    return y * s;
-}
-
 // KUNIT: the argument is known >= 0.0038 (non-negative linear RGB).
 template <bool KUNIT>
 __device__ __forceinline__ float opsin_row(int g, float r, float gg, float b) {
@@ -331,22 +276,6 @@ __device__ __forceinline__ float xyb_from_opsin(int g, float rg, float gr, float
     if (g == 0) return fmaf(0.5f * (rg - gr), 14.0f, 0.42f);
     if (g == 1) return y + 0.01f;
     return (bb - y) + 0.55f;
-}
-
-// BT.709 inverse OETF (crates/cuda-colorspace-kernel/src/lib.rs:223-238):
-// ((v + (alpha - 1)) / alpha)^(1/0.45) above the threshold, v / 4.5 below.
-// The two divisions are multiplications by the f32 reciprocals 1/alpha and
-// 2/9 (<= 1 ulp from dividing); both branches are evaluated and selected.
-// The power's base is clamped to [1/8, 1.5]: the selected branch has
-// base >= 0.164, and a base above 1.5 (v > 1.55, possible only for NV12,
-// whose caller clamps the result to 1) gives a result above 1 either way.
-__device__ __forceinline__ float bt709_eotf(float v) {
-    const float alpha_m1 = 0x1.96b84p-4f;    // alpha - 1, alpha = 1 + 5.5 * 0.018053968510807
-    const float inv_alpha = 0x1.d1c096p-1f;  // 1 / alpha in f32
-    const float thr = 0.08124285829863521110029445797874f;
-    const float hi = s2_pow_20_9_unit(fminf(fmaxf((v + alpha_m1) * inv_alpha, 0.125f), 1.5f));
-    const float lo = v * 0x1.c71c72p-3f;     // v / 4.5
-    return v >= thr ? hi : lo;
 }
 
 // ---- two pixels at once (sm_100 f32x2 operations; each lane rounds exactly
@@ -402,11 +331,6 @@ __device__ __forceinline__ void ds_lab2(float2 r, float2 g, float2 b, float2 o[3
     o[2] = __ffma2_rn(__fadd2_rn(fy, s2_neg2(fz)), s2_f2(200.0f / 220.0f), s2_f2(107.9f / 220.0f));
 }
 
-
-__device__ __forceinline__ float s2_pow_scale_unit(unsigned b) {
-    const int e = (int)(b >> 23) - 127;
-    return e == 0 ? 1.0f : (e == -1 ? 0x1.b6e8aep-3f : (e == -2 ? 0x1.784086p-5f : 0x1.428a3p-7f));
-}
 
 // Packed f32x2 arithmetic (__fmul2_rn, __fadd2_rn, __ffma2_rn): each lane
 // rounds as the scalar operation, but the compiler contracts a packed
@@ -464,14 +388,39 @@ __device__ __forceinline__ float2 s2_div2_neg(float2 a, float2 b) {
     return s2_pfma(e, r, q);
 }
 
-// The factors 2^(20e/9) of s2_pow_20_9_unit for e = -3..0, indexed by the
-// exponent field minus 124 (the caller keeps them in shared memory: one
-// shared load per lane instead of three compares and selects).
-#define S2_POW_TAB_INIT {0x1.428a3p-7f, 0x1.784086p-5f, 0x1.b6e8aep-3f, 0x1p+0f}
+// BT.709 inverse OETF (crates/cuda-colorspace-kernel/src/lib.rs:223-238) of
+// two samples: ((v + (alpha - 1)) / alpha)^(1/0.45) from the threshold on,
+// v / 4.5 below; the two divisions are multiplications by the f32 reciprocals
+// 1/alpha and 2/9 (<= 1 ulp from dividing), and both branches are evaluated and
+// selected.  p^(1/0.45) = p^(20/9) with p = m 2^e, m in [1, 2): m^(20/9) is a
+// degree-7 polynomial in t = m - 1.5 (Chebyshev interpolation at 8 nodes,
+// converted to monomials and rounded to f32; Horner with fmaf), times
+// 2^(20e/9), one f32 constant per exponent (a power of two times a rounded
+// 2^(r/9)); <= 3.3 ulp on [0.1, 2].
+//
+// pw: s2_pow_table() of every exponent field, sign bit included, so that no
+// value needs a clamp before the lookup: the selected branch has p >= 0.164
+// (e >= -3), and where p >= 2 the factor only has to give a result above 1.
+//
+// SAT: the result clamped to [0, 1] (the 4:2:0 family), which the last
+// multiplications do for nothing.  Without SAT the power's base is clamped to
+// [1/8, 1.5], its value for samples beyond the nominal range.
+constexpr int kPowTable = 512;
+__host__ __device__ __forceinline__ float s2_pow_table(int field) {
+    return field < 124 || field > 255 ? 0.0f
+                                      : (field > 127 ? 4.0f
+                                                     : (field == 127 ? 1.0f
+                                                                     : (field == 126 ? 0x1.b6e8aep-3f
+                                                                                     : (field == 125 ? 0x1.784086p-5f : 0x1.428a3p-7f))));
+}
 
-// s2_pow_20_9_unit of both lanes; pw = the S2_POW_TAB_INIT table
-__device__ __forceinline__ float2 s2_pow_20_9_unit2(float2 p, const float *pw) {
-    const unsigned bx = __float_as_uint(p.x), by = __float_as_uint(p.y);
+template <bool SAT>
+__device__ __forceinline__ float2 bt709_eotf2(float2 v, const float *pw) {
+    const float thr = 0.08124285829863521110029445797874f;
+    // alpha - 1 and 1 / alpha, alpha = 1 + 5.5 * 0.018053968510807
+    float2 q = s2_mul2(s2_add2(v, s2_f2(0x1.96b84p-4f)), s2_f2(0x1.d1c096p-1f));
+    if (!SAT) q = make_float2(fminf(fmaxf(q.x, 0.125f), 1.5f), fminf(fmaxf(q.y, 0.125f), 1.5f));
+    const unsigned bx = __float_as_uint(q.x), by = __float_as_uint(q.y);
     const float2 m = make_float2(__uint_as_float((bx & 0x7fffffu) | 0x3f800000u),
                                  __uint_as_float((by & 0x7fffffu) | 0x3f800000u));
     const float2 t = s2_add2(m, s2_f2(-1.5f));
@@ -482,16 +431,13 @@ __device__ __forceinline__ float2 s2_pow_20_9_unit2(float2 p, const float *pw) {
     y = __ffma2_rn(y, t, s2_f2(0x1.7c6f02p+0f));
     y = __ffma2_rn(y, t, s2_f2(0x1.d2e55cp+1f));
     y = __ffma2_rn(y, t, s2_f2(0x1.3b279ep+1f));
-    return s2_mul2(y, make_float2(pw[(bx >> 23) - 124u], pw[(by >> 23) - 124u]));
-}
-
-// bt709_eotf of both lanes; pw = the S2_POW_TAB_INIT table
-__device__ __forceinline__ float2 bt709_eotf2(float2 v, const float *pw) {
-    const float thr = 0.08124285829863521110029445797874f;
-    const float2 q = s2_mul2(s2_add2(v, s2_f2(0x1.96b84p-4f)), s2_f2(0x1.d1c096p-1f));
-    const float2 hi =
-        s2_pow_20_9_unit2(make_float2(fminf(fmaxf(q.x, 0.125f), 1.5f), fminf(fmaxf(q.y, 0.125f), 1.5f)), pw);
-    const float2 lo = s2_mul2(v, s2_f2(0x1.c71c72p-3f));
+    const float fx = pw[bx >> 23], fy = pw[by >> 23], slope = 0x1.c71c72p-3f;
+    if (SAT) {
+        const float hx = __saturatef(y.x * fx), hy = __saturatef(y.y * fy);
+        const float lx = __saturatef(v.x * slope), ly = __saturatef(v.y * slope);
+        return make_float2(v.x >= thr ? hx : lx, v.y >= thr ? hy : ly);
+    }
+    const float2 hi = s2_mul2(y, make_float2(fx, fy)), lo = s2_mul2(v, s2_f2(slope));
     return make_float2(v.x >= thr ? hi.x : lo.x, v.y >= thr ? hi.y : lo.y);
 }
 
@@ -502,11 +448,13 @@ __device__ __forceinline__ float2 s2_cbrtf_unit2(float2 x) {
     float2 y = s2_mul2(x, r);
     y = s2_mul2(y, r);
     const float2 hi = s2_mul2(y, y);
-    const float2 lo = __ffma2_rn(y, y, s2_neg2(hi));
-    float2 e = __ffma2_rn(hi, y, s2_neg2(x));
+    // the two subtractions as scalar FMAs, whose operands negate for nothing
+    // (a packed operand takes a logic instruction per lane to negate)
+    const float2 lo = make_float2(fmaf(y.x, y.x, -hi.x), fmaf(y.y, y.y, -hi.y));
+    float2 e = make_float2(fmaf(hi.x, y.x, -x.x), fmaf(hi.y, y.y, -x.y));
     e = __ffma2_rn(lo, y, e);
-    const float2 c = s2_mul2(s2_mul2(r, r), s2_f2(0x1.555556p-2f));
-    return __ffma2_rn(s2_neg2(e), c, y);
+    const float2 nc = s2_mul2(s2_mul2(r, r), s2_f2(-0x1.555556p-2f));
+    return __ffma2_rn(e, nc, y);
 }
 
 // XYB of two pixels of non-negative linear RGB (opsin_row<true> and
@@ -523,27 +471,16 @@ __device__ __forceinline__ void xyb_pair_unit(float2 r, float2 g, float2 b, floa
     const float2 gr = s2_add2(s2_cbrtf_unit2(v1), nroot);
     const float2 bb = s2_add2(s2_cbrtf_unit2(v2), nroot);
     const float2 y = s2_mul2(s2_f2(0.5f), s2_add2(rg, gr));
-    out[0] = __ffma2_rn(s2_mul2(s2_f2(0.5f), s2_add2(rg, s2_neg2(gr))), s2_f2(14.0f), s2_f2(0.42f));
+    // a - b as b * -1 + a: one rounding, that of the subtraction
+    out[0] = __ffma2_rn(s2_mul2(s2_f2(0.5f), __ffma2_rn(gr, s2_f2(-1.0f), rg)), s2_f2(14.0f), s2_f2(0.42f));
     out[1] = s2_add2(y, s2_f2(0.01f));
-    out[2] = s2_add2(s2_add2(bb, s2_neg2(y)), s2_f2(0.55f));
+    out[2] = s2_add2(__ffma2_rn(y, s2_f2(-1.0f), bb), s2_f2(0.55f));
 }
 
 struct ColorConsts {
     // BT.2020 -> BT.709 linear matrix (row-major)
     float m2020[9];
 };
-
-__device__ __forceinline__ void rgb16_linear(unsigned r, unsigned g, unsigned b, float inv, const ColorConsts &cc,
-                                             float o[3]) {
-    const float p0 = bt709_eotf((float)r * inv);
-    const float p1 = bt709_eotf((float)g * inv);
-    const float p2 = bt709_eotf((float)b * inv);
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-        const float *m = cc.m2020 + 3 * k;
-        o[k] = fmaxf(fmaf(m[0], p0, fmaf(m[1], p1, m[2] * p2)), 0.0f);
-    }
-}
 
 template <typename T> __device__ __forceinline__ float ld_store(const T *p);
 template <> __device__ __forceinline__ float ld_store<float>(const float *p) { return __ldg(p); }
@@ -558,33 +495,35 @@ template <> __device__ __forceinline__ __nv_bfloat16 to_store<__nv_bfloat16>(flo
     return __float2bfloat16_rn(v);
 }
 
-// RGB16: samples of `bits` bits, BT.709/BT.2020 inverse OETF, then BT.2020 ->
-// BT.709 primaries, clamped >= 0.  inv = 1 / (2^bits - 1) in f32.
-struct ColorConsts;
-__device__ __forceinline__ void rgb16_linear(unsigned r, unsigned g, unsigned b, float inv, const ColorConsts &cc,
-                                             float o[3]);
+// A 2x2 quad of linear RGB: [row][channel], lanes = left and right pixel.
+struct Quad {
+    float2 c[2][3];
+};
 
-// Linear RGB of scale-0 pixel (x, y) of image img (inside the image), for
-// input format FMT (the packed formats; 4:2:0 YUV goes by whole quads,
-// yuv_load_quad / yuv_quad_linear).  sRGB8: the reference table; RGB16:
-// BT.709/BT.2020 inverse OETF, then BT.2020 -> BT.709 primaries, clamped >= 0.
-template <int FMT>
-__device__ __forceinline__ void lin_pixel(const DevPair &P, int img, int x, int y, const float *lut,
-                                          const ColorConsts &cc, float o[3]) {
-    const char *base = (const char *)P.in[img] + (long long)y * P.pitch[img];
-    if (FMT == FMT_LINEAR_F32) {
-        const float *q = (const float *)base + 3 * x;
-        o[0] = __ldg(q);
-        o[1] = __ldg(q + 1);
-        o[2] = __ldg(q + 2);
-    } else if (FMT == FMT_SRGB8) {
-        const uint8_t *q = (const uint8_t *)base + 3 * x;
-        o[0] = lut[__ldg(q)];
-        o[1] = lut[__ldg(q + 1)];
-        o[2] = lut[__ldg(q + 2)];
-    } else {
-        const uint16_t *q = (const uint16_t *)base + 3 * x;
-        rgb16_linear(__ldg(q), __ldg(q + 1), __ldg(q + 2), 1.0f / (float)((1 << P.bits) - 1), cc, o);
+// Sample `i` (0 low half, 1 high half) of a word of two samples of ES bytes,
+// plus 2^23, as a float: the sample is the float's low mantissa bits, and
+// subtracting 2^23 (exact) leaves it (a conversion would go through the SFU).
+template <int ES>
+__device__ __forceinline__ float s2_sample(unsigned w, int i) {
+    return __uint_as_float(__byte_perm(w, 0x4b000000u, ES == 1 ? (i ? 0x7441 : 0x7440) : (i ? 0x7432 : 0x7410)));
+}
+constexpr float kSample0 = 8388608.0f;
+
+// RGB16: two pixels (words lo: r0 g0, mid: b0 r1, hi: g1 b1) of samples of
+// `bits` bits, BT.709/BT.2020 inverse OETF, then BT.2020 -> BT.709 primaries,
+// clamped >= 0.  inv = 1 / (2^bits - 1) in f32.  The scaled samples are scalar
+// products: the OETF adds to them.
+__device__ __forceinline__ void rgb16_linear2(unsigned lo, unsigned mid, unsigned hi, float inv, const ColorConsts &cc,
+                                              const float *pw, float2 o[3]) {
+    const float2 r = make_float2((s2_sample<2>(lo, 0) - kSample0) * inv, (s2_sample<2>(mid, 1) - kSample0) * inv);
+    const float2 g = make_float2((s2_sample<2>(lo, 1) - kSample0) * inv, (s2_sample<2>(hi, 0) - kSample0) * inv);
+    const float2 b = make_float2((s2_sample<2>(mid, 0) - kSample0) * inv, (s2_sample<2>(hi, 1) - kSample0) * inv);
+    const float2 p0 = bt709_eotf2<false>(r, pw), p1 = bt709_eotf2<false>(g, pw), p2 = bt709_eotf2<false>(b, pw);
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const float *m = cc.m2020 + 3 * k;
+        const float2 v = __ffma2_rn(s2_f2(m[0]), p0, __ffma2_rn(s2_f2(m[1]), p1, __fmul2_rn(s2_f2(m[2]), p2)));
+        o[k] = make_float2(fmaxf(v.x, 0.0f), fmaxf(v.y, 0.0f));
     }
 }
 
@@ -619,91 +558,83 @@ __device__ __forceinline__ Nv12Quad yuv_load_quad(const DevPair &P, int img, int
 
 // Limited / full range YUV of the pair's matrix (cuda-colorspace-kernel/src/
 // biplanar.rs:8-70: nearest chroma, luma floored at the range minimum, BT.709
-// inverse OETF, clamp to [0, 1]) of a loaded quad: pixels (0, 1) and (2, 3)
-// as f32x2 lanes.
+// inverse OETF, clamp to [0, 1]) of a loaded quad.
 template <int ES>
-__device__ __forceinline__ void yuv_quad_linear(const Nv12Quad &q, const DevPair &P, const float *pw, float o[4][3]) {
-    constexpr unsigned kMask = ES == 1 ? 0xffu : 0xffffu;
-    constexpr int kShift = 8 * ES;
-    const float cb = (float)((int)(q.uv & kMask) - P.yuv_neutral);
-    const float cr = (float)((int)(q.uv >> kShift) - P.yuv_neutral);
+__device__ __forceinline__ void yuv_quad_linear(const Nv12Quad &q, const DevPair &P, const float *pw, Quad &o) {
+    const float neutral = kSample0 + (float)P.yuv_neutral, ymin = kSample0 + (float)P.yuv_min, yc = P.yuv[0];
+    const float cb = s2_sample<ES>(q.uv, 0) - neutral, cr = s2_sample<ES>(q.uv, 1) - neutral;
     const float ar = P.yuv[1] * cr;
     const float ag = fmaf(P.yuv[3], cb, P.yuv[4] * cr);
     const float ab = P.yuv[2] * cb;
-    const int ymin = P.yuv_min;
-    const float yc = P.yuv[0];
 #pragma unroll
     for (int row = 0; row < 2; row++) {
         const unsigned w = row ? q.y1 : q.y0;
-        const int Y0 = (int)(w & kMask), Y1 = (int)(w >> kShift);
         // scalar products: luma is summed with the chroma terms below
-        const float2 luma = make_float2((float)(max(Y0, ymin) - ymin) * yc, (float)(max(Y1, ymin) - ymin) * yc);
-        const float2 r = bt709_eotf2(s2_add2(luma, s2_f2(ar)), pw);
-        const float2 g = bt709_eotf2(s2_add2(luma, s2_f2(ag)), pw);
-        const float2 b = bt709_eotf2(s2_add2(luma, s2_f2(ab)), pw);
-        float *p0 = o[2 * row], *p1 = o[2 * row + 1];
-        p0[0] = fminf(fmaxf(r.x, 0.0f), 1.0f);
-        p0[1] = fminf(fmaxf(g.x, 0.0f), 1.0f);
-        p0[2] = fminf(fmaxf(b.x, 0.0f), 1.0f);
-        p1[0] = fminf(fmaxf(r.y, 0.0f), 1.0f);
-        p1[1] = fminf(fmaxf(g.y, 0.0f), 1.0f);
-        p1[2] = fminf(fmaxf(b.y, 0.0f), 1.0f);
+        const float2 luma = make_float2(fmaxf(s2_sample<ES>(w, 0) - ymin, 0.0f) * yc,
+                                        fmaxf(s2_sample<ES>(w, 1) - ymin, 0.0f) * yc);
+        o.c[row][0] = bt709_eotf2<true>(s2_add2(luma, s2_f2(ar)), pw);
+        o.c[row][1] = bt709_eotf2<true>(s2_add2(luma, s2_f2(ag)), pw);
+        o.c[row][2] = bt709_eotf2<true>(s2_add2(luma, s2_f2(ab)), pw);
     }
 }
 
 // Linear RGB of the 2x2 quad whose top-left pixel is (x, y) (inside the
-// image); px 0..3 = (x,y), (x+1,y), (x,y+1), (x+1,y+1); pixels outside the
-// image (vx / vy false) are not read.  NV12 chroma is one sample per quad.
-// lut: the sRGB8 table (256 entries) followed by the S2_POW_TAB_INIT table.
+// image) for the packed formats.  A column or row outside the image (vx / vy
+// false) is not read: it repeats the left pixel, the upper row.  lut: the
+// sRGB8 table; pw: the s2_pow_table.
 template <int FMT>
-__device__ __forceinline__ void lin_quad(const DevPair &P, int img, int x, int y, bool vx, bool vy,
-                                         const float *lut, const ColorConsts &cc, float o[4][3]) {
-    if (FMT == FMT_NV12 || FMT == FMT_P016) {
-        // 4:2:0 input has even width and height: the quad is complete
-        constexpr int ES = FMT == FMT_NV12 ? 1 : 2;
-        yuv_quad_linear<ES>(yuv_load_quad<ES>(P, img, x, y), P, lut + 256, o);
-    } else {
-        // a complete quad whose rows are aligned for the format's word size is
-        // read as three words per row: sRGB8 16-bit, RGB16 32-bit, linear f32
-        // 64-bit (x is even: the row pair starts 6, 12 or 24 bytes x/2 in)
-        constexpr int kAlign = FMT == FMT_SRGB8 ? 2 : (FMT == FMT_RGB16 ? 4 : 8);
-        if (vx && vy && ((((unsigned long long)P.in[img]) | (unsigned long long)P.pitch[img]) & (kAlign - 1)) == 0) {
-            const float inv = FMT == FMT_RGB16 ? 1.0f / (float)((1 << P.bits) - 1) : 0.0f;
+__device__ __forceinline__ void lin_quad(const DevPair &P, int img, int x, int y, bool vx, bool vy, const float *lut,
+                                         const float *pw, const ColorConsts &cc, Quad &o) {
+    // a complete row of the quad whose rows are aligned for the format's word
+    // size is read as three words: sRGB8 16-bit, RGB16 32-bit, linear f32
+    // 64-bit (x is even: the row pair starts 6, 12 or 24 bytes x/2 in)
+    constexpr int kAlign = FMT == FMT_SRGB8 ? 2 : (FMT == FMT_RGB16 ? 4 : 8);
+    const bool words = vx && ((((unsigned long long)P.in[img]) | (unsigned long long)P.pitch[img]) & (kAlign - 1)) == 0;
+    const float inv = FMT == FMT_RGB16 ? 1.0f / (float)((1 << P.bits) - 1) : 0.0f;
+    const int right = vx ? 3 : 0;  // samples from the left pixel to the right one
 #pragma unroll
-            for (int row = 0; row < 2; row++) {
-                const char *rp = (const char *)P.in[img] + (long long)(y + row) * P.pitch[img];
-                float *p0 = o[2 * row], *p1 = o[2 * row + 1];
-                if (FMT == FMT_SRGB8) {
-                    const unsigned short *q = (const unsigned short *)(rp + 3 * x);
-                    const unsigned w0 = __ldg(q), w1 = __ldg(q + 1), w2 = __ldg(q + 2);
-                    p0[0] = lut[w0 & 0xffu];
-                    p0[1] = lut[w0 >> 8];
-                    p0[2] = lut[w1 & 0xffu];
-                    p1[0] = lut[w1 >> 8];
-                    p1[1] = lut[w2 & 0xffu];
-                    p1[2] = lut[w2 >> 8];
-                } else if (FMT == FMT_RGB16) {
-                    const unsigned *q = (const unsigned *)(rp + 6 * x);
-                    const unsigned w0 = __ldg(q), w1 = __ldg(q + 1), w2 = __ldg(q + 2);
-                    rgb16_linear(w0 & 0xffffu, w0 >> 16, w1 & 0xffffu, inv, cc, p0);
-                    rgb16_linear(w1 >> 16, w2 & 0xffffu, w2 >> 16, inv, cc, p1);
-                } else {
-                    const float2 *q = (const float2 *)(rp + 12 * x);
-                    const float2 a = __ldg(q), b = __ldg(q + 1), c = __ldg(q + 2);
-                    p0[0] = a.x;
-                    p0[1] = a.y;
-                    p0[2] = b.x;
-                    p1[0] = b.y;
-                    p1[1] = c.x;
-                    p1[2] = c.y;
-                }
+    for (int row = 0; row < 2; row++) {
+        const char *rp = (const char *)P.in[img] + (long long)(y + (vy ? row : 0)) * P.pitch[img];
+        if (FMT == FMT_SRGB8) {
+            unsigned w0, w1, w2;
+            if (words) {
+                const unsigned short *q = (const unsigned short *)(rp + 3 * x);
+                w0 = __ldg(q), w1 = __ldg(q + 1), w2 = __ldg(q + 2);
+            } else {
+                const uint8_t *q = (const uint8_t *)rp + 3 * x;
+                w0 = __ldg(q) | (unsigned)__ldg(q + 1) << 8;
+                w1 = __ldg(q + 2) | (unsigned)__ldg(q + right) << 8;
+                w2 = __ldg(q + right + 1) | (unsigned)__ldg(q + right + 2) << 8;
             }
+            o.c[row][0] = make_float2(lut[w0 & 0xffu], lut[w1 >> 8]);
+            o.c[row][1] = make_float2(lut[w0 >> 8], lut[w2 & 0xffu]);
+            o.c[row][2] = make_float2(lut[w1 & 0xffu], lut[w2 >> 8]);
+        } else if (FMT == FMT_RGB16) {
+            unsigned w0, w1, w2;
+            if (words) {
+                const unsigned *q = (const unsigned *)(rp + 6 * x);
+                w0 = __ldg(q), w1 = __ldg(q + 1), w2 = __ldg(q + 2);
+            } else {
+                const uint16_t *q = (const uint16_t *)rp + 3 * x;
+                w0 = __ldg(q) | (unsigned)__ldg(q + 1) << 16;
+                w1 = __ldg(q + 2) | (unsigned)__ldg(q + right) << 16;
+                w2 = __ldg(q + right + 1) | (unsigned)__ldg(q + right + 2) << 16;
+            }
+            rgb16_linear2(w0, w1, w2, inv, cc, pw, o.c[row]);
         } else {
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-                const bool in = (k & 1 ? vx : true) && (k & 2 ? vy : true);
-                if (in) lin_pixel<FMT>(P, img, x + (k & 1), y + (k >> 1), lut, cc, o[k]);
+            float2 a, b, c;
+            if (words) {
+                const float2 *q = (const float2 *)(rp + 12 * x);
+                a = __ldg(q), b = __ldg(q + 1), c = __ldg(q + 2);
+            } else {
+                const float *q = (const float *)rp + 3 * x;
+                a = make_float2(__ldg(q), __ldg(q + 1));
+                b = make_float2(__ldg(q + 2), __ldg(q + right));
+                c = make_float2(__ldg(q + right + 1), __ldg(q + right + 2));
             }
+            o.c[row][0] = make_float2(a.x, b.y);
+            o.c[row][1] = make_float2(a.y, c.x);
+            o.c[row][2] = make_float2(b.x, c.y);
         }
     }
 }

@@ -118,30 +118,37 @@ __device__ __forceinline__ void store_xyb(const DevPair &P, int img, int s, int 
     for (int c = 0; c < 3; c++) dst[c * plane + off] = to_store<ST>(o[c]);
 }
 
-// XYB of two horizontally adjacent pixels, stored as one 2-element write
-// (x even: the planes' pitch is a multiple of 64 elements).
-template <typename ST, bool KUNIT>
-__device__ __forceinline__ void store_xyb_pair(ST *dst, long long plane, long long off, const float a[3],
-                                               const float b[3]) {
-    float2 o[3];
+// XYB of two pixels (lanes).
+template <bool KUNIT>
+__device__ __forceinline__ void xyb_pair(const float2 l[3], float2 o[3]) {
     if (KUNIT) {
-        xyb_pair_unit(make_float2(a[0], b[0]), make_float2(a[1], b[1]), make_float2(a[2], b[2]), o);
+        xyb_pair_unit(l[0], l[1], l[2], o);
     } else {
+        const float a[3] = {l[0].x, l[1].x, l[2].x}, b[3] = {l[0].y, l[1].y, l[2].y};
         float oa[3], ob[3];
         xyb3<KUNIT>(a, oa);
         xyb3<KUNIT>(b, ob);
 #pragma unroll
         for (int c = 0; c < 3; c++) o[c] = make_float2(oa[c], ob[c]);
     }
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-        if constexpr (sizeof(ST) == 4) {
-            *(float2 *)(dst + c * plane + off) = o[c];
-        } else {
-            ST two[2] = {to_store<ST>(o[c].x), to_store<ST>(o[c].y)};
-            *(unsigned *)(dst + c * plane + off) = *(const unsigned *)two;
-        }
+}
+
+// The first n of the values a.x, a.y, b.x, b.y from d on (d 16-byte aligned:
+// a multiple of four columns in a plane whose pitch is a multiple of 64).
+__device__ __forceinline__ void store4(float *d, float2 a, float2 b, int n) {
+    if (n >= 4) {
+        *(float4 *)d = make_float4(a.x, a.y, b.x, b.y);
+    } else {
+        d[0] = a.x;
+        if (n > 1) d[1] = a.y;
+        if (n > 2) d[2] = b.x;
     }
+}
+
+// Two from d on (8-byte aligned), or one.
+__device__ __forceinline__ void store2(float *d, float2 a, bool two) {
+    if (two) *(float2 *)d = a;
+    else d[0] = a.x;
 }
 
 // DSSIM outputs of one level's pixel: its Lab (levels below lab_levels) and,
@@ -163,29 +170,32 @@ __device__ __forceinline__ void store_lab(const DevPair &P, int img, int s, int 
     }
 }
 
-// The same for pixels (x, y) and, when `two`, (x + 1, y) of one row, their
-// Lab formed two at a time (ds_lab2, each lane as ds_lab).
-__device__ __forceinline__ void store_lab_pair(const DevPair &P, int img, int s, int x, int y, const float a[3],
-                                               const float b[3], bool two) {
+// The same for a row of pixels formed as pairs: N = 2 pairs from a multiple of
+// four columns on, or N = 1 pair from an even one; n pixels are inside the level.
+template <int N>
+__device__ __forceinline__ void store_lab_row(const DevPair &P, int img, int s, int x, int y, const float2 (*l)[3],
+                                              int n) {
     const long long plane = (long long)P.lp[s] * P.h[s];
     const long long off = (long long)y * P.lp[s] + x;
     if (s < P.lab_levels) {
-        float2 o[3];
-        ds_lab2(make_float2(a[0], two ? b[0] : a[0]), make_float2(a[1], two ? b[1] : a[1]),
-                make_float2(a[2], two ? b[2] : a[2]), o);
-        float *dst = P.lab[img][s];
+        float2 o[N][3];
+#pragma unroll
+        for (int k = 0; k < N; k++) ds_lab2(l[k][0], l[k][1], l[k][2], o[k]);
+        float *dst = P.lab[img][s] + off;
 #pragma unroll
         for (int c = 0; c < 3; c++) {
-            dst[c * plane + off] = o[c].x;
-            if (two) dst[c * plane + off + 1] = o[c].y;
+            if (N == 2) store4(dst, o[0][c], o[N - 1][c], n);
+            else store2(dst, o[0][c], n > 1);
+            dst += plane;
         }
     }
     if (s == P.lab_levels - 1 && P.keep[img]) {
-        float *dst = P.keep[img];
+        float *dst = P.keep[img] + off;
 #pragma unroll
         for (int c = 0; c < 3; c++) {
-            dst[c * plane + off] = a[c];
-            if (two) dst[c * plane + off + 1] = b[c];
+            if (N == 2) store4(dst, l[0][c], l[N - 1][c], n);
+            else store2(dst, l[0][c], n > 1);
+            dst += plane;
         }
     }
 }
@@ -194,14 +204,20 @@ __device__ __forceinline__ void store_lab_pair(const DevPair &P, int img, int s,
 // the same linear pyramid).  OUT == 1 is the SSIMULACRA2-only pass.
 //
 // A thread takes two horizontally adjacent 2x2 quads at a time (4 x 2
-// scale-0 pixels): the scale-0 XYB goes out as pixel pairs, and the two
-// quads' scale-1 pixels form one pair for the f32x2 XYB conversion too.
+// scale-0 pixels) as pixel pairs: a row's XYB goes out as 16-byte words, and
+// the two quads' scale-1 pixels form one pair for the f32x2 XYB conversion too.
+// Pixels of a quad outside the image repeat the left pixel and the upper row
+// (downscale.rs:4-35's clamped source) and are not stored.
+//
+// What bounds it: instructions of colour arithmetic (per pixel 3 BT.709 powers
+// and 3 cube roots, with another 1/3 of the cube roots for the smaller
+// scales).  @Q@
 //
 // BLK: the block's edge.  A block of kPyrBlk converts both images; one of
 // kPyrBlkSmall converts `only` one.
 template <int FMT, typename ST, int OUT, int BLK>
-__device__ __forceinline__ void prep_quads(const DevPair &P, int X0, int Y0, const float *lut, const ColorConsts &cc,
-                                           float (*lv1)[3][BLK / 2 * (BLK / 2)], int only) {
+__device__ __forceinline__ void prep_quads(const DevPair &P, int X0, int Y0, const float *lut, const float *pw,
+                                           const ColorConsts &cc, float (*lv1)[3][BLK / 2 * (BLK / 2)], int only) {
     constexpr int kLv1 = BLK / 2;  // scale-1 block edge
     constexpr bool kOne = BLK == kPyrBlkSmall;
     const int mask = kOne ? 1 << only : P.prep_mask;
@@ -209,6 +225,7 @@ __device__ __forceinline__ void prep_quads(const DevPair &P, int X0, int Y0, con
     constexpr bool kX = (OUT & 1) != 0, kL = (OUT & 2) != 0;
     constexpr bool kYuv = FMT == FMT_NV12 || FMT == FMT_P016;
     constexpr int kEs = FMT == FMT_P016 ? 2 : 1;
+    static_assert(sizeof(ST) == 4, "f32 planes");
     const int W = P.w[0], H = P.h[0];
     const bool scale1 = (kL ? P.prep_levels : P.nscales) > 1;
     for (int qq = threadIdx.x; qq < kLv1 * kLv1 / 2; qq += blockDim.x) {
@@ -232,58 +249,72 @@ __device__ __forceinline__ void prep_quads(const DevPair &P, int X0, int Y0, con
 #pragma unroll 1
         for (int img = kOne ? only : 0; img < (kOne ? only + 1 : 2); img++) {
             if (!kOne && !((mask >> img) & 1)) continue;
-            float l1[2][3];
+            Quad q[2];
+            if (kYuv) {
+                yuv_quad_linear<kEs>(img ? nd0 : nr0, P, pw, q[0]);
+                yuv_quad_linear<kEs>(img ? nd1 : nr1, P, pw, q[1]);
+            } else {
+                lin_quad<FMT>(P, img, x, y, x + 1 < W, vy, lut, pw, cc, q[0]);
+                lin_quad<FMT>(P, img, two ? x + 2 : x, y, x + 3 < W, vy, lut, pw, cc, q[1]);
+            }
+            if (kX && (!kL || P.nscales > 0)) {
+                const long long plane = (long long)P.lp[0] * H;
+                float *dst = (float *)P.lvl[img][0] + (long long)y * P.lp[0] + x;
 #pragma unroll
-            for (int k = 0; k < 2; k++) {
-                if (k == 1 && !two) break;
-                const int xq = x + 2 * k;
-                const bool vx = xq + 1 < W;
-                float v[4][3];
-                if (kYuv) yuv_quad_linear<kEs>(img ? (k ? nd1 : nd0) : (k ? nr1 : nr0), P, lut + 256, v);
-                else lin_quad<FMT>(P, img, xq, y, vx, vy, lut, cc, v);
-                if (kX && (!kL || P.nscales > 0)) {
-                    ST *dst = (ST *)P.lvl[img][0];
-                    const long long plane = (long long)P.lp[0] * H;
-                    const long long off = (long long)y * P.lp[0] + xq;
-                    if (vx) store_xyb_pair<ST, KU>(dst, plane, off, v[0], v[1]);
-                    else store_xyb<ST, KU>(P, img, 0, xq, y, v[0]);
-                    if (vy) {
-                        if (vx) store_xyb_pair<ST, KU>(dst, plane, off + P.lp[0], v[2], v[3]);
-                        else store_xyb<ST, KU>(P, img, 0, xq, y + 1, v[2]);
+                for (int row = 0; row < 2; row++) {
+                    if (row && !vy) break;
+                    float2 o0[3], o1[3];
+                    xyb_pair<KU>(q[0].c[row], o0);
+                    xyb_pair<KU>(q[1].c[row], o1);
+                    float *d = dst;
+#pragma unroll
+                    for (int c = 0; c < 3; c++) {
+                        store4(d, o0[c], o1[c], W - x);
+                        d += plane;
                     }
+                    dst += P.lp[0];
                 }
-                if (kL) {
-                    store_lab_pair(P, img, 0, xq, y, v[0], v[1], vx);
-                    if (vy) store_lab_pair(P, img, 0, xq, y + 1, v[2], v[3], vx);
-                }
-                // scale-1 pixel: 2x2 mean, far-edge clamp (a missing column
-                // repeats the left pixel, a missing row the upper one)
+            }
+            if (kL) {
 #pragma unroll
-                for (int c = 0; c < 3; c++) {
-                    const float a = v[0][c];
-                    const float b = vx ? v[1][c] : a;
-                    const float cc2 = vy ? v[2][c] : a;
-                    const float d = vy ? (vx ? v[3][c] : cc2) : b;
-                    float sum = a + b;
-                    sum = sum + cc2;
-                    sum = sum + d;
-                    l1[k][c] = sum * 0.25f;
+                for (int row = 0; row < 2; row++) {
+                    if (row && !vy) break;
+                    float2 l[2][3];
+#pragma unroll
+                    for (int c = 0; c < 3; c++) l[0][c] = q[0].c[row][c], l[1][c] = q[1].c[row][c];
+                    store_lab_row<2>(P, img, 0, x, y + row, l, W - x);
                 }
             }
             if (!scale1) continue;
+            // scale-1 pixels: 2x2 means
+            float2 l1[1][3];
             const int x1 = (X0 >> 1) + qx, y1 = (Y0 >> 1) + qy;
 #pragma unroll
             for (int c = 0; c < 3; c++) {
-                lv1[kOne ? 0 : img][c][qy * kLv1 + qx] = l1[0][c];
-                if (two) lv1[kOne ? 0 : img][c][qy * kLv1 + qx + 1] = l1[1][c];
+                float m[2];
+#pragma unroll
+                for (int k = 0; k < 2; k++) {
+                    float sum = q[k].c[0][c].x + q[k].c[0][c].y;
+                    sum = sum + q[k].c[1][c].x;
+                    sum = sum + q[k].c[1][c].y;
+                    m[k] = sum * 0.25f;
+                }
+                l1[0][c] = make_float2(m[0], m[1]);
+                *(float2 *)&lv1[kOne ? 0 : img][c][qy * kLv1 + qx] = l1[0][c];
             }
             if (kX && (!kL || P.nscales > 1)) {
                 // x1 is even and the planes' pitch a multiple of 64 elements
-                if (two) store_xyb_pair<ST, KU>((ST *)P.lvl[img][1], (long long)P.lp[1] * P.h[1],
-                                                (long long)y1 * P.lp[1] + x1, l1[0], l1[1]);
-                else store_xyb<ST, KU>(P, img, 1, x1, y1, l1[0]);
+                const long long plane = (long long)P.lp[1] * P.h[1];
+                float *d = (float *)P.lvl[img][1] + (long long)y1 * P.lp[1] + x1;
+                float2 o[3];
+                xyb_pair<KU>(l1[0], o);
+#pragma unroll
+                for (int c = 0; c < 3; c++) {
+                    store2(d, o[c], two);
+                    d += plane;
+                }
             }
-            if (kL) store_lab_pair(P, img, 1, x1, y1, l1[0], l1[1], two);
+            if (kL) store_lab_row<1>(P, img, 1, x1, y1, l1, two ? 2 : 1);
         }
     }
 }
@@ -314,18 +345,19 @@ __global__ void __launch_bounds__(kPrepThreads, 4) prep_kernel(const DevPair *__
     if (zero && blockIdx.x == 0 && threadIdx.x < kCounterInts) zero[threadIdx.x] = 0;
     constexpr int kLv1 = BLK / 2;
     constexpr int kImgs = BLK == kPyrBlkSmall ? 1 : 2;        // images of a block
-    __shared__ float lv1[kImgs][3][kLv1 * kLv1];              // scale-1 linear block [img][ch][px]
+    __shared__ __align__(8) float lv1[kImgs][3][kLv1 * kLv1];  // scale-1 linear block [img][ch][px]
     __shared__ float pp[2][kImgs][3][(kLv1 / 2) * (kLv1 / 2)];  // scales >= 2, ping-pong
-    __shared__ float lut[256 + 4];  // the sRGB8 table, then the BT.709 power's 2^(20e/9) factors
+    constexpr bool kLut = FMT < 0 || FMT == FMT_SRGB8, kPow = FMT < 0 || (FMT != FMT_SRGB8 && FMT != FMT_LINEAR_F32);
+    __shared__ float lut[kLut ? 256 : 1];     // the sRGB8 table
+    __shared__ float pw[kPow ? kPowTable : 1];  // the BT.709 power's 2^(20e/9) factors
     // the block's pair descriptor: in shared memory, so the level stores
     // (global) cannot alias it and its fields need no per-thread copy
     __shared__ DevPair sP;
     static_assert(sizeof(DevPair) % 8 == 0, "DevPair copied as 8-byte words");
-    for (int i = threadIdx.x; i < 256; i += blockDim.x) lut[i] = lut_g[i];
-    if (threadIdx.x < 4) {
-        const float pw[4] = S2_POW_TAB_INIT;
-        lut[256 + threadIdx.x] = pw[threadIdx.x];
-    }
+    if (kLut)
+        for (int i = threadIdx.x; i < 256; i += blockDim.x) lut[i] = lut_g[i];
+    if (kPow)
+        for (int i = threadIdx.x; i < kPowTable; i += blockDim.x) pw[i] = s2_pow_table(i);
     const int items = (end_block - first_block) * (2 / kImgs);
     for (int it = blockIdx.x; it < items; it += gridDim.x) {
         const int item = first_block + (kImgs == 1 ? it >> 1 : it);
@@ -346,14 +378,14 @@ __global__ void __launch_bounds__(kPrepThreads, 4) prep_kernel(const DevPair *__
         const int bx = b % P.blk_x, by = b / P.blk_x;
         const int X0 = bx * BLK, Y0 = by * BLK;
         if constexpr (FMT >= 0) {
-            prep_quads<(FMT >= 0 ? FMT : 0), ST, OUT, BLK>(P, X0, Y0, lut, cc, lv1, only);
+            prep_quads<(FMT >= 0 ? FMT : 0), ST, OUT, BLK>(P, X0, Y0, lut, pw, cc, lv1, only);
         } else {
             switch (P.fmt) {
-            case FMT_LINEAR_F32: prep_quads<FMT_LINEAR_F32, ST, OUT, BLK>(P, X0, Y0, lut, cc, lv1, only); break;
-            case FMT_SRGB8: prep_quads<FMT_SRGB8, ST, OUT, BLK>(P, X0, Y0, lut, cc, lv1, only); break;
-            case FMT_NV12: prep_quads<FMT_NV12, ST, OUT, BLK>(P, X0, Y0, lut, cc, lv1, only); break;
-            case FMT_P016: prep_quads<FMT_P016, ST, OUT, BLK>(P, X0, Y0, lut, cc, lv1, only); break;
-            default: prep_quads<FMT_RGB16, ST, OUT, BLK>(P, X0, Y0, lut, cc, lv1, only); break;
+            case FMT_LINEAR_F32: prep_quads<FMT_LINEAR_F32, ST, OUT, BLK>(P, X0, Y0, lut, pw, cc, lv1, only); break;
+            case FMT_SRGB8: prep_quads<FMT_SRGB8, ST, OUT, BLK>(P, X0, Y0, lut, pw, cc, lv1, only); break;
+            case FMT_NV12: prep_quads<FMT_NV12, ST, OUT, BLK>(P, X0, Y0, lut, pw, cc, lv1, only); break;
+            case FMT_P016: prep_quads<FMT_P016, ST, OUT, BLK>(P, X0, Y0, lut, pw, cc, lv1, only); break;
+            default: prep_quads<FMT_RGB16, ST, OUT, BLK>(P, X0, Y0, lut, pw, cc, lv1, only); break;
             }
         }
         __syncthreads();
