@@ -40,3 +40,22 @@ def test_small_and_large_blocks_agree(tmb, cuda, fmt, w, h):
     assert alone[0] == both[0] and alone[5] == both[5]
     for k in (1, 2, 6):
         assert np.array_equal(alone[k], both[k])
+
+
+@pytest.mark.parametrize("w,h", [(8, 8), (9, 11), (33, 34), (66, 65), (131, 70)])
+@pytest.mark.parametrize("left,pitch", [(0, 0), (1, 1), (2, 5), (3, 2)])
+def test_rows_at_any_byte(tmb, cuda, w, h, left, pitch):
+    """sRGB8 rows that start at any byte (crops, odd widths) are read in whole
+    words; the statistics are those of a packed, aligned copy, bit for bit."""
+    ref, dis = synth.srgb_pair(w + left + pitch, h, 33, 12)
+    crops = [cuda.from_numpy(a).cuda()[:, left:left + w] for a in (ref, dis)]
+    s = tmb.Ssimulacra2(w, h, strip_rows=32)
+    s.compute_srgb(*crops)
+    got = s.get_result()
+    # 64 pixels of padding a row: every row starts at a multiple of 4 bytes
+    wide = [cuda.zeros((h, (w + 67) // 4 * 4, 3), dtype=cuda.uint8, device="cuda") for _ in crops]
+    for a, c in zip(wide, crops):
+        a[:, :w] = c
+    s.compute_srgb(*(a[:, :w] for a in wide))
+    want = s.get_result()
+    assert got[0] == want[0] and np.array_equal(got[1], want[1]) and np.array_equal(got[2], want[2])

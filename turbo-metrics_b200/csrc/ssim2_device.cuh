@@ -401,29 +401,30 @@ __device__ __forceinline__ float2 s2_div2_neg(float2 a, float2 b) {
 // pw: s2_pow_table() of every exponent field, sign bit included, so that no
 // value needs a clamp before the lookup: the selected branch has p >= 0.164
 // (e >= -3), and where p >= 2 the factor only has to give a result above 1.
+// An entry also holds 2^-e, which turns p into m in the multiply-add that
+// forms t (exact; picking m's bits out of p took a logic instruction more).
 //
 // SAT: the result clamped to [0, 1] (the 4:2:0 family), which the last
 // multiplications do for nothing.  Without SAT the power's base is clamped to
 // [1/8, 1.5], its value for samples beyond the nominal range.
 constexpr int kPowTable = 512;
-__host__ __device__ __forceinline__ float s2_pow_table(int field) {
-    return field < 124 || field > 255 ? 0.0f
-                                      : (field > 127 ? 4.0f
-                                                     : (field == 127 ? 1.0f
-                                                                     : (field == 126 ? 0x1.b6e8aep-3f
-                                                                                     : (field == 125 ? 0x1.784086p-5f : 0x1.428a3p-7f))));
+__host__ __device__ __forceinline__ float2 s2_pow_table(int field) {
+    if (field < 124 || field > 255) return make_float2(0.0f, 0.0f);
+    if (field > 127) return make_float2(4.0f, 0.5f);
+    return field == 127 ? make_float2(1.0f, 1.0f)
+                        : (field == 126 ? make_float2(0x1.b6e8aep-3f, 2.0f)
+                                        : (field == 125 ? make_float2(0x1.784086p-5f, 4.0f)
+                                                        : make_float2(0x1.428a3p-7f, 8.0f)));
 }
 
 template <bool SAT>
-__device__ __forceinline__ float2 bt709_eotf2(float2 v, const float *pw) {
+__device__ __forceinline__ float2 bt709_eotf2(float2 v, const float2 *pw) {
     const float thr = 0.08124285829863521110029445797874f;
     // alpha - 1 and 1 / alpha, alpha = 1 + 5.5 * 0.018053968510807
     float2 q = s2_mul2(s2_add2(v, s2_f2(0x1.96b84p-4f)), s2_f2(0x1.d1c096p-1f));
     if (!SAT) q = make_float2(fminf(fmaxf(q.x, 0.125f), 1.5f), fminf(fmaxf(q.y, 0.125f), 1.5f));
-    const unsigned bx = __float_as_uint(q.x), by = __float_as_uint(q.y);
-    const float2 m = make_float2(__uint_as_float((bx & 0x7fffffu) | 0x3f800000u),
-                                 __uint_as_float((by & 0x7fffffu) | 0x3f800000u));
-    const float2 t = s2_add2(m, s2_f2(-1.5f));
+    const float2 fx = pw[__float_as_uint(q.x) >> 23], fy = pw[__float_as_uint(q.y) >> 23];
+    const float2 t = make_float2(fmaf(q.x, fx.y, -1.5f), fmaf(q.y, fy.y, -1.5f));
     float2 y = __ffma2_rn(s2_f2(0x1.1eb37ap-12f), t, s2_f2(-0x1.88e318p-11f));
     y = __ffma2_rn(y, t, s2_f2(0x1.2713a6p-9f));
     y = __ffma2_rn(y, t, s2_f2(-0x1.37717ep-7f));
@@ -431,20 +432,25 @@ __device__ __forceinline__ float2 bt709_eotf2(float2 v, const float *pw) {
     y = __ffma2_rn(y, t, s2_f2(0x1.7c6f02p+0f));
     y = __ffma2_rn(y, t, s2_f2(0x1.d2e55cp+1f));
     y = __ffma2_rn(y, t, s2_f2(0x1.3b279ep+1f));
-    const float fx = pw[bx >> 23], fy = pw[by >> 23], slope = 0x1.c71c72p-3f;
+    const float slope = 0x1.c71c72p-3f;
     if (SAT) {
-        const float hx = __saturatef(y.x * fx), hy = __saturatef(y.y * fy);
+        const float hx = __saturatef(y.x * fx.x), hy = __saturatef(y.y * fy.x);
         const float lx = __saturatef(v.x * slope), ly = __saturatef(v.y * slope);
         return make_float2(v.x >= thr ? hx : lx, v.y >= thr ? hy : ly);
     }
-    const float2 hi = s2_mul2(y, make_float2(fx, fy)), lo = s2_mul2(v, s2_f2(slope));
+    const float2 hi = make_float2(y.x * fx.x, y.y * fy.x), lo = s2_mul2(v, s2_f2(slope));
     return make_float2(v.x >= thr ? hi.x : lo.x, v.y >= thr ? hi.y : lo.y);
 }
 
 // s2_cbrtf_unit of both lanes (each lane rounds as the scalar steps: no
 // packed product feeds a packed sum)
 __device__ __forceinline__ float2 s2_cbrtf_unit2(float2 x) {
-    const float2 r = make_float2(s2_rcbrt_sfu(x.x), s2_rcbrt_sfu(x.y));
+    float2 l, r;  // s2_rcbrt_sfu of both lanes
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(l.x) : "f"(x.x));
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(l.y) : "f"(x.y));
+    l = s2_mul2(l, s2_f2(-0x1.555556p-2f));
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r.x) : "f"(l.x));
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r.y) : "f"(l.y));
     float2 y = s2_mul2(x, r);
     y = s2_mul2(y, r);
     const float2 hi = s2_mul2(y, y);
@@ -514,7 +520,7 @@ constexpr float kSample0 = 8388608.0f;
 // clamped >= 0.  inv = 1 / (2^bits - 1) in f32.  The scaled samples are scalar
 // products: the OETF adds to them.
 __device__ __forceinline__ void rgb16_linear2(unsigned lo, unsigned mid, unsigned hi, float inv, const ColorConsts &cc,
-                                              const float *pw, float2 o[3]) {
+                                              const float2 *pw, float2 o[3]) {
     const float2 r = make_float2((s2_sample<2>(lo, 0) - kSample0) * inv, (s2_sample<2>(mid, 1) - kSample0) * inv);
     const float2 g = make_float2((s2_sample<2>(lo, 1) - kSample0) * inv, (s2_sample<2>(hi, 0) - kSample0) * inv);
     const float2 b = make_float2((s2_sample<2>(mid, 0) - kSample0) * inv, (s2_sample<2>(hi, 1) - kSample0) * inv);
@@ -560,7 +566,7 @@ __device__ __forceinline__ Nv12Quad yuv_load_quad(const DevPair &P, int img, int
 // biplanar.rs:8-70: nearest chroma, luma floored at the range minimum, BT.709
 // inverse OETF, clamp to [0, 1]) of a loaded quad.
 template <int ES>
-__device__ __forceinline__ void yuv_quad_linear(const Nv12Quad &q, const DevPair &P, const float *pw, Quad &o) {
+__device__ __forceinline__ void yuv_quad_linear(const Nv12Quad &q, const DevPair &P, const float2 *pw, Quad &o) {
     const float neutral = kSample0 + (float)P.yuv_neutral, ymin = kSample0 + (float)P.yuv_min, yc = P.yuv[0];
     const float cb = s2_sample<ES>(q.uv, 0) - neutral, cr = s2_sample<ES>(q.uv, 1) - neutral;
     const float ar = P.yuv[1] * cr;
@@ -584,7 +590,7 @@ __device__ __forceinline__ void yuv_quad_linear(const Nv12Quad &q, const DevPair
 // sRGB8 table; pw: the s2_pow_table.
 template <int FMT>
 __device__ __forceinline__ void lin_quad(const DevPair &P, int img, int x, int y, bool vx, bool vy, const float *lut,
-                                         const float *pw, const ColorConsts &cc, Quad &o) {
+                                         const float2 *pw, const ColorConsts &cc, Quad &o) {
     // a complete row of the quad whose rows are aligned for the format's word
     // size is read as three words: sRGB8 16-bit, RGB16 32-bit, linear f32
     // 64-bit (x is even: the row pair starts 6, 12 or 24 bytes x/2 in)

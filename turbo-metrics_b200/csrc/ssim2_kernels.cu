@@ -100,10 +100,10 @@ __device__ __forceinline__ int find_seg(const Seg *segs, int nseg, int tile, int
 // ---------------------------------------------------------------------------
 // prep: input -> linear -> XYB of every scale (2x2 box pyramid in linear RGB)
 //
-// Block = 64x64 scale-0 pixels of one pair, 256 threads, each thread a 2x2
-// quad at a time: it converts the quad's four pixels, stores their XYB, and
-// averages them (downscale.rs:4-35, source clamped at the far edge) into the
-// scale-1 pixel, whose XYB it stores too and whose linear RGB goes to shared
+// Block = 64x64 (or 32x32) scale-0 pixels of one pair, each thread two 2x2
+// quads at a time: it converts their eight pixels, stores their XYB, and
+// averages each quad (downscale.rs:4-35, source clamped at the far edge) into
+// a scale-1 pixel, whose XYB it stores too and whose linear RGB goes to shared
 // memory for scales 2..5.
 // ---------------------------------------------------------------------------
 // KUNIT: linear RGB known non-negative (every input format but linear f32).
@@ -118,7 +118,8 @@ __device__ __forceinline__ void store_xyb(const DevPair &P, int img, int s, int 
     for (int c = 0; c < 3; c++) dst[c * plane + off] = to_store<ST>(o[c]);
 }
 
-// XYB of two pixels (lanes).
+// XYB of two pixels (lanes).  KUNIT: linear RGB known non-negative (every
+// input format but linear f32).
 template <bool KUNIT>
 __device__ __forceinline__ void xyb_pair(const float2 l[3], float2 o[3]) {
     if (KUNIT) {
@@ -170,8 +171,10 @@ __device__ __forceinline__ void store_lab(const DevPair &P, int img, int s, int 
     }
 }
 
-// The same for a row of pixels formed as pairs: N = 2 pairs from a multiple of
-// four columns on, or N = 1 pair from an even one; n pixels are inside the level.
+// DSSIM outputs of one level's row of pixels formed as pairs: their Lab (levels
+// below lab_levels) and, for the clamp pass, their linear RGB (level
+// lab_levels - 1, when kept).  N = 2 pairs from a multiple of four columns on,
+// or N = 1 pair from an even one; n pixels are inside the level.
 template <int N>
 __device__ __forceinline__ void store_lab_row(const DevPair &P, int img, int s, int x, int y, const float2 (*l)[3],
                                               int n) {
@@ -211,12 +214,19 @@ __device__ __forceinline__ void store_lab_row(const DevPair &P, int img, int s, 
 //
 // What bounds it: instructions of colour arithmetic (per pixel 3 BT.709 powers
 // and 3 cube roots, with another 1/3 of the cube roots for the smaller
-// scales).  @Q@
+// scales).  Per submission (B200), before the conversions ran on pixel pairs
+// throughout, with table entries for every exponent instead of clamps, free
+// saturation and negation, and 16-byte stores -> now: 64 x 1080p NV12 1810 ->
+// 1508 us, 64 uneven sRGB8 pairs 1021 -> 825, 4 x 3840x2160 RGB16 (whose
+// powers were scalar) 746 -> 465, 16 x 720p P016 with Lab 501 -> 412.  Tried
+// and slower: sRGB8 rows as shifted 32-bit words (880), levels 2..5 as pixel
+// pairs in unrolled code (897), the two rows' cube roots in one rolled loop
+// (943, sRGB8), five blocks per SM (864, sRGB8).
 //
 // BLK: the block's edge.  A block of kPyrBlk converts both images; one of
 // kPyrBlkSmall converts `only` one.
 template <int FMT, typename ST, int OUT, int BLK>
-__device__ __forceinline__ void prep_quads(const DevPair &P, int X0, int Y0, const float *lut, const float *pw,
+__device__ __forceinline__ void prep_quads(const DevPair &P, int X0, int Y0, const float *lut, const float2 *pw,
                                            const ColorConsts &cc, float (*lv1)[3][BLK / 2 * (BLK / 2)], int only) {
     constexpr int kLv1 = BLK / 2;  // scale-1 block edge
     constexpr bool kOne = BLK == kPyrBlkSmall;
@@ -346,10 +356,10 @@ __global__ void __launch_bounds__(kPrepThreads, 4) prep_kernel(const DevPair *__
     constexpr int kLv1 = BLK / 2;
     constexpr int kImgs = BLK == kPyrBlkSmall ? 1 : 2;        // images of a block
     __shared__ __align__(8) float lv1[kImgs][3][kLv1 * kLv1];  // scale-1 linear block [img][ch][px]
-    __shared__ float pp[2][kImgs][3][(kLv1 / 2) * (kLv1 / 2)];  // scales >= 2, ping-pong
+    __shared__ __align__(8) float pp[2][kImgs][3][(kLv1 / 2) * (kLv1 / 2)];  // scales >= 2, ping-pong
     constexpr bool kLut = FMT < 0 || FMT == FMT_SRGB8, kPow = FMT < 0 || (FMT != FMT_SRGB8 && FMT != FMT_LINEAR_F32);
     __shared__ float lut[kLut ? 256 : 1];     // the sRGB8 table
-    __shared__ float pw[kPow ? kPowTable : 1];  // the BT.709 power's 2^(20e/9) factors
+    __shared__ float2 pw[kPow ? kPowTable : 1];  // the BT.709 power's 2^(20e/9) factors
     // the block's pair descriptor: in shared memory, so the level stores
     // (global) cannot alias it and its fields need no per-thread copy
     __shared__ DevPair sP;
@@ -391,12 +401,14 @@ __global__ void __launch_bounds__(kPrepThreads, 4) prep_kernel(const DevPair *__
         __syncthreads();
         const int nlev = (OUT & 2) ? P.prep_levels : P.nscales;
         for (int s = 2; s < nlev; s++) {
+            constexpr int kLog = BLK == 64 ? 6 : 5;
+            static_assert(BLK == 1 << kLog, "block edge");
             const int bs = BLK >> s, pbs = BLK >> (s - 1);
             const int ox0 = X0 >> s, oy0 = Y0 >> s;
             const int px0 = X0 >> (s - 1), py0 = Y0 >> (s - 1);
             const int wp = P.w[s - 1], hp = P.h[s - 1];
             for (int i = threadIdx.x; i < bs * bs; i += blockDim.x) {
-                const int ox = ox0 + i % bs, oy = oy0 + i / bs;
+                const int ox = ox0 + (i & (bs - 1)), oy = oy0 + (i >> (kLog - s));
                 if (ox >= P.w[s] || oy >= P.h[s]) continue;
                 // downscale.rs:4-35: source index clamped to the previous level
                 const int xa = 2 * ox, xb = min(2 * ox + 1, wp - 1);
@@ -416,7 +428,7 @@ __global__ void __launch_bounds__(kPrepThreads, 4) prep_kernel(const DevPair *__
                         pp[s & 1][at][c][i] = v[c];
                     }
                     if ((OUT & 1) && (!(OUT & 2) || s < P.nscales)) {
-                        if (P.fmt == FMT_LINEAR_F32) store_xyb<ST, false>(P, img, s, ox, oy, v);
+                        if (FMT == FMT_LINEAR_F32 || (FMT < 0 && P.fmt == FMT_LINEAR_F32)) store_xyb<ST, false>(P, img, s, ox, oy, v);
                         else store_xyb<ST, true>(P, img, s, ox, oy, v);
                     }
                     if (OUT & 2) store_lab(P, img, s, ox, oy, v);
