@@ -872,7 +872,7 @@ struct Engine {
         if (profiling) S2_CUDA(cudaEventRecord(prof[2], st));
         if (m_s2)
             S2_CUDA(launch_finalize(dpairs, n, (const double *)partials_d.p, err_word(), results_at(n), st,
-                                    !split && blur != S2_BLUR_IIR_REF));
+                                    !split));
         if (profiling) S2_CUDA(cudaEventRecord(prof[3], st));
         if (m_ds) S2_CUDA(launch_ds(P, dbase, st));
         if (profiling) S2_CUDA(cudaEventRecord(prof[4], st));
@@ -940,7 +940,7 @@ struct Engine {
         }
         if (e == cudaSuccess && m_s2)
             e = launch_finalize(dpairs, n, (const double *)partials_d.p, err_word(), results_at(n), cap_st,
-                                blur != S2_BLUR_IIR_REF);
+                                true);
         if (e == cudaSuccess && m_ds) e = launch_ds(P, dbase, cap_st);
         if (e == cudaSuccess && results_at(n) != results_h)
             e = cudaMemcpyAsync(results_h, results_d.p, n * sizeof(DevResult), cudaMemcpyDeviceToHost, cap_st);

@@ -36,6 +36,7 @@
 // reference, with the engine's own cube root); finalize_kernel reduces the row
 // records in order.  The translation unit is compiled with -fmad=false: every
 // FMA below is explicit, as in the reference (Rust never contracts).
+#include "dependent_launch.cuh"
 #include "ssim2_device.cuh"
 #include "ssim2_launch.h"
 
@@ -186,6 +187,7 @@ __global__ void __launch_bounds__(kHThreads, 2) iir_horizontal_kernel(const DevP
                                                              double *__restrict__ partials) {
     extern __shared__ __align__(16) float hsm[];
     __shared__ double red[kHelpers][6];
+    dep::grid_wait();  // the vertical walk is done
     const IirSeg sg = segs[find_iseg(segs, nseg, blockIdx.x)];
     const DevPair &P = pairs[sg.pair];
     const int s = sg.scale, W = P.w[s], H = P.h[s], lp = P.lp[s];
@@ -331,13 +333,13 @@ cudaError_t launch_iir(int storage, const DevPair *pairs, const IirSeg *vsegs, i
                        const IirSeg *hsegs, int nhseg, int htotal, double *partials, cudaStream_t st) {
     (void)storage;  // f32 planes only
     if (vtotal > 0) {
-        iir_vertical_kernel<float><<<vtotal, kVThreads, 0, st>>>(pairs, vsegs, nvseg);
-        cudaError_t e = cudaGetLastError();
+        const cudaError_t e =
+            dep::launch(false, iir_vertical_kernel<float>, dim3(vtotal), kVThreads, 0, st, pairs, vsegs, nvseg);
         if (e != cudaSuccess) return e;
     }
     if (htotal > 0) {
-        iir_horizontal_kernel<float><<<htotal, kHThreads, kHSmem, st>>>(pairs, hsegs, nhseg, partials);
-        return cudaGetLastError();
+        return dep::launch(true, iir_horizontal_kernel<float>, dim3(htotal), kHThreads, kHSmem, st, pairs, hsegs, nhseg,
+                           partials);
     }
     return cudaSuccess;
 }

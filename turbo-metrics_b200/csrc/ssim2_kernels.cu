@@ -28,19 +28,17 @@
 // algebraically (including at image borders, where the blur of a constant is
 // not the constant).
 #include "../../include/ssim2b200.h"
+#include "dependent_launch.cuh"
 #include "ssim2_device.cuh"
 #include "ssim2_launch.h"
 
 namespace s2 {
 
-// Programmatic dependent launch: a kernel launched with it starts as soon as
-// the blocks of the one before it in the stream have all started (they say so
-// first thing), sets itself up, and waits here until that one is complete.
-// With the counters zeroed by the prep pass and a few pairs' results stored
-// straight to host memory, a 96x64 pair's call went from 47.3 to 34.4 us and a
-// 1920x1080 one's from 131 to 119 (three graph nodes and two launch latencies).
-__device__ __forceinline__ void s2_grid_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void s2_grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// The tile pass and finalize launch dependently (dependent_launch.cuh).  With
+// the counters zeroed by the prep pass and a few pairs' results stored straight
+// to host memory, a 96x64 pair's call went from 47.3 to 34.4 us and a 1920x1080
+// one's from 131 to 119 (three graph nodes and two launch latencies).
+
 
 // Shared memory of fused_kernel (one CTA = one channel of a tile): the step
 // buffer, three float2 planes of kStep rows x kRS columns -- plane 0 and 1
@@ -350,7 +348,6 @@ __global__ void __launch_bounds__(kPrepThreads, 4) prep_kernel(const DevPair *__
                                                    int end_block,
                                                    ColorConsts cc, const float *__restrict__ lut_g,
                                                    int *__restrict__ zero) {
-    s2_grid_start();
     // the tile pass's work counters and time-out word, for the pass that follows
     if (zero && blockIdx.x == 0 && threadIdx.x < kCounterInts) zero[threadIdx.x] = 0;
     constexpr int kLv1 = BLK / 2;
@@ -945,8 +942,7 @@ __global__ void __launch_bounds__(kFusedThreads, kTileBlocks)
         s_bad = 0;
         s2_wait_limit = ck.wait_cycles;
     }
-    s2_grid_start();
-    s2_grid_wait();  // the planes are written
+    dep::grid_wait();  // the planes are written
     __syncthreads();
     unsigned phase = 0;
     int item = first_item + blockIdx.x;  // the grid is at most the items
@@ -991,7 +987,7 @@ __global__ void __launch_bounds__(kFinThreads) finalize_kernel(const DevPair *__
                                                                DevResult *__restrict__ out) {
     __shared__ double red[kFinGroups][108];
     __shared__ double st[108];
-    s2_grid_wait();  // the tile records are written
+    dep::grid_wait();  // the tile records are written
     const int p = blockIdx.x;
     const DevPair &P = pairs[p];
     const int t = threadIdx.x, g = t / 18, j = t % 18;
@@ -1175,23 +1171,6 @@ cudaError_t launch_pyramid(int storage, const DevPair *pairs, int npairs, const 
     return cudaGetLastError();
 }
 
-// Launch with or without programmatic dependence on the kernel before it.
-template <typename... Params, typename... Args>
-static cudaError_t launch_after(bool early, void (*kernel)(Params...), int grid, int block, size_t smem, cudaStream_t st,
-                                Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr = {};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = early ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
-}
-
 cudaError_t launch_fused(int storage, const DevPair *pairs, const Seg *segs, int nseg, int first_tile, int end_tile,
                          int *counter, const TileCheck &ck, double *partials, int grid, cudaStream_t st, bool early) {
     const int fi = 3 * first_tile, ei = 3 * end_tile;  // work items: (tile, channel)
@@ -1199,7 +1178,7 @@ cudaError_t launch_fused(int storage, const DevPair *pairs, const Seg *segs, int
     if (nt <= 0) return cudaSuccess;
     grid = grid > nt ? nt : grid;
     (void)storage;
-    return launch_after(early, fused_kernel<float, false>, grid, kTileThreads, fused_smem_bytes(), st, pairs, segs, nseg,
+    return dep::launch(early, fused_kernel<float, false>, dim3(grid), kTileThreads, fused_smem_bytes(), st, pairs, segs, nseg,
                         fi, ei, counter, ck, partials, MapOut{nullptr, 0, 0});
 }
 
@@ -1233,7 +1212,7 @@ cudaError_t launch_desc_copy(void *dst, const void *src_host_mapped, size_t byte
 cudaError_t launch_finalize(const DevPair *pairs, int npairs, const double *partials, const int *err,
                             DevResult *out, cudaStream_t st, bool early) {
     if (npairs <= 0) return cudaSuccess;
-    return launch_after(early, finalize_kernel, npairs, kFinThreads, 0, st, pairs, npairs, partials, err, out);
+    return dep::launch(early, finalize_kernel, dim3(npairs), kFinThreads, 0, st, pairs, npairs, partials, err, out);
 }
 
 }  // namespace s2

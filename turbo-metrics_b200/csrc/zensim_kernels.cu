@@ -40,6 +40,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "dependent_launch.cuh"
 #include "zensim_kernels.h"
 
 namespace zs {
@@ -234,6 +235,7 @@ constexpr int kWalkThreads = 128 + kChunk * (kZsWalkW / 4);
 
 __global__ void __launch_bounds__(kWalkThreads, 3) zs_walk_kernel(const __grid_constant__ ZsPlan plan) {
     extern __shared__ __align__(16) float smem[];
+    dep::grid_wait();  // both pyramids are written
     float(*ring)[kRingRows][kZsWalkW] = (float(*)[kRingRows][kZsWalkW])smem;
     int s = 0;
     while (s + 1 < plan.ns && (int)blockIdx.x >= plan.sc[s + 1].walk_first) s++;
@@ -332,6 +334,7 @@ __global__ void __launch_bounds__(kFeatThreads, 3) zs_feat_kernel(const __grid_c
     const size_t pitch = S.ref.pitch;
     const float *A = S.ref.p[ch], *D = S.dis.p[ch];
     const int ybase = y0 - kZsRadius;
+    dep::grid_wait();  // the saved sums are written
     for (int i = t; i < kFeatRows * (kZsTileW / 4); i += kFeatThreads) {
         const int r = i / (kZsTileW / 4), c = 4 * (i % (kZsTileW / 4)), x = x0 + c, y = ybase + r;
         if (x >= n || y < 0 || y >= h) continue;
@@ -460,6 +463,7 @@ __global__ void __launch_bounds__(kZsOut *kRuns) zs_reduce_kernel(const __grid_c
                                                                   const double *__restrict__ in,
                                                                   double *__restrict__ out) {
     __shared__ double red[kRuns][kZsOut];
+    dep::grid_wait();
     const ZsScale &S = plan.sc[blockIdx.x / 3];
     const int per = S.tiles_x * S.tiles_y, t = threadIdx.x, i = t % kZsOut, r = t / kZsOut;
     const double *q = in + ((size_t)S.tile_first + (size_t)(blockIdx.x % 3) * per) * kZsOut + i;
@@ -492,10 +496,12 @@ cudaError_t zs_launch_prep(const uint8_t *img, size_t pitch, int w, int h, const
 }
 
 cudaError_t zs_launch_features(const ZsPlan &plan, double *tile_out, double *out, cudaStream_t st) {
-    zs_walk_kernel<<<plan.walk_blocks, kWalkThreads, kWalkSmem, st>>>(plan);
-    zs_feat_kernel<<<plan.tiles, kFeatThreads, kFeatSmem, st>>>(plan, tile_out);
-    zs_reduce_kernel<<<plan.ns * 3, kZsOut * kRuns, 0, st>>>(plan, tile_out, out);
-    return cudaGetLastError();
+    cudaError_t e = dep::launch(true, zs_walk_kernel, dim3(plan.walk_blocks), kWalkThreads, kWalkSmem, st, plan);
+    if (e == cudaSuccess)
+        e = dep::launch(true, zs_feat_kernel, dim3(plan.tiles), kFeatThreads, kFeatSmem, st, plan, tile_out);
+    if (e == cudaSuccess)
+        e = dep::launch(true, zs_reduce_kernel, dim3(plan.ns * 3), kZsOut * kRuns, 0, st, plan, tile_out, out);
+    return e;
 }
 
 }  // namespace zs
