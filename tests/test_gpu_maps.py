@@ -65,3 +65,23 @@ def test_error_maps_preconditions(tmb, cuda):
     t.get_score()
     with pytest.raises(tmb.S2Error):
         t.error_maps(0)
+
+
+@pytest.mark.parametrize("w,h", [(120, 16), (121, 33), (1921, 1601), (3841, 1701)])
+def test_maps_in_every_tile_height_pool_to_the_statistics(tmb, cuda, w, h):
+    """The export's own tiles are 16, 32 or 64 rows high, by the size of the
+    scale: in each the maps of scale 0 give back the compute's statistics."""
+    g = cuda.Generator(device="cuda")
+    g.manual_seed(w)
+    ref = cuda.randint(0, 256, (h, w, 3), generator=g, device="cuda", dtype=cuda.uint8)
+    dis = (ref // 16 * 16 + 8).clamp(0, 255).to(cuda.uint8)
+    s = tmb.Ssimulacra2(w, h)
+    s.compute_srgb(ref, dis)
+    _, stats, _ = s.get_result()
+    m = s.error_maps(0).double()
+    l1 = m.mean((2, 3)).cpu().numpy()
+    l4 = (m ** 4).mean((2, 3)).cpu().numpy() ** 0.25
+    for c in range(3):
+        want = stats[c * 36:c * 36 + 6]
+        assert np.all(np.abs(l1[c] - want[:3]) <= 1e-5 * want[:3] + 1e-9), (c, l1[c], want)
+        assert np.all(np.abs(l4[c] - want[3:]) <= 1e-5 * want[3:] + 1e-9), (c, l4[c], want)

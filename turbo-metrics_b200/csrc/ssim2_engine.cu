@@ -731,18 +731,23 @@ s2_status s2_error_maps(s2_ctx *ctx, int32_t scale, float *maps, size_t pitch, v
     if (p.status != S2_OK || scale < 0 || scale >= p.nscales) return S2_ERR_INVALID_ARG;
     const size_t row = (size_t)p.w[scale] * sizeof(float);
     if (pitch < row || pitch % sizeof(float)) return S2_ERR_DIM_MISMATCH;
-    // the last compute's descriptors and XYB planes are still in the
-    // workspace; re-run its tile pass over this scale with the export on
-    const int t0 = p.tile_base[scale], t1 = t0 + p.tile_cnt[scale];
-    const size_t pb = s2_align_up(sizeof(DevPair), 256), bb = s2_align_up(sizeof(int), 256);
-    char *dbase = (char *)e.pairs_d.p;
+    // the last compute's descriptor and XYB planes are still in the workspace;
+    // re-run the tile pass over this scale with the export on, in tiles as tall
+    // as leave about four waves of (tile, channel) items, like the planner's
+    Seg seg = {};
+    seg.scale = scale;
+    seg.tiles_x = (p.w[scale] + kTileW - 1) / kTileW;
+    int tiles = 0;
+    for (int rows : {kStripMax, kStripMid, kStripMin}) {
+        seg.strip_rows = rows;
+        tiles = seg.tiles_x * ((p.h[scale] + rows - 1) / rows);
+        if (3 * tiles >= 4 * e.num_sms * e.fused_bps) break;
+    }
     cudaStream_t st = (cudaStream_t)stream;
     const long long mpitch = (long long)(pitch / sizeof(float));
     S2_CUDA(cudaMemsetAsync(e.counter_d.p, 0, Engine::kCounterBytes, st));
-    S2_CUDA(launch_fused_export(e.storage, (const DevPair *)dbase, (const Seg *)(dbase + pb + bb),
-                                (int)P.segs.size(), t0, t1, (int *)e.counter_d.p, tile_check(e.err_word()),
-                                (double *)e.partials_d.p, maps, mpitch, mpitch * p.h[scale], e.num_sms * e.fused_bps,
-                                st));
+    S2_CUDA(launch_fused_export((const DevPair *)e.pairs_d.p, seg, tiles, (int *)e.counter_d.p,
+                                tile_check(e.err_word()), maps, mpitch, mpitch * p.h[scale], e.num_sms, st));
     // the tile pass's time-out word (set only if its row copies never landed)
     int err = 0;
     S2_CUDA(cudaMemcpyAsync(&err, e.err_word(), sizeof err, cudaMemcpyDeviceToHost, st));

@@ -479,10 +479,17 @@ __global__ void __launch_bounds__(kPrepThreads, 4) prep_kernel(const DevPair *__
 //
 // EXPORT (error-map export, one scale of one pair): every pixel's SSIM error,
 // artifact and detail-loss values are also stored to `maps`, 9 planes
-// [channel][map] of `mpitch` floats per row and `mplane` floats per plane.
+// [channel][map] of `mpitch` floats per row and `mplane` floats per plane.  A
+// step's values go through shared memory, so that a warp stores 32 adjacent
+// floats of a row: the tasks, whose lanes are 8 rows and 4 segments apart,
+// stored 32 sectors at a time.  Scale 0 of 1023x769: 57 us with those stores
+// and the compute's 64-row tiles (351 blocks), 39 now.
+// The export has a segment of its own (tiles of the height that suits one
+// scale alone; the maps do not depend on it) and keeps no sums.
 struct MapOut {
     float *maps;
     long long mpitch, mplane;
+    Seg seg;
 };
 
 // Register rings of one vertical column.
@@ -700,11 +707,26 @@ __device__ __forceinline__ void add_task(double *a, const TaskSums &ts) {
     a[5 * kFusedThreads] += (double)ts.f4_ad.y;
 }
 
+// A step's map values on their way out (EXPORT): [map][row][column].
+constexpr int kExpRow = kTileW + 1, kExpMap = kStep * kExpRow;
+
+// The maps of the step's rows r0 .. r0 + nr - 1, a row of a map per warp.
+__device__ __forceinline__ void export_rows(const float *__restrict__ ebuf, int r0, int nr, const ItemGeo &G,
+                                            const MapOut &mo, int tid) {
+    const int cols = min(kTileW, G.W - G.x0);
+    for (int i = tid >> 5; i < 3 * nr; i += kFusedThreads / 32) {
+        const int map = i / nr, r = i - map * nr;
+        const float *s = ebuf + map * kExpMap + r * kExpRow;
+        float *d = mo.maps + (3 * G.g + map) * mo.mplane + (long long)(G.y0 + r0 + r) * mo.mpitch + G.x0;
+        for (int x = tid & 31; x < cols; x += 32) d[x] = s[x];
+    }
+}
+
 // Horizontal phase of one step (output rows r0 .. r0 + nr - 1 of the tile):
 // this thread's task, row t_r, segment t_s; its sums are added to acc.
 template <bool EXPORT, typename ACC>
 __device__ __forceinline__ void h_step(const float2 *__restrict__ buf, int r0, int nr, int t_r, int t_s, bool t_on,
-                                       const ItemGeo &G, ACC &&acc, const MapOut &mo) {
+                                       const ItemGeo &G, ACC &&acc, float *__restrict__ ebuf) {
     if (!t_on || t_r >= nr) return;
     const int c0 = t_s * kSegW;  // first output column of the task (tile coordinates)
     const int xc = G.x0 + c0;
@@ -734,10 +756,10 @@ __device__ __forceinline__ void h_step(const float2 *__restrict__ buf, int r0, i
                 float d, art, det;
                 maps_px<false>(mA[j], mB[j], rw[j], 0.0f, 0.0f, d, art, det);
                 if (EXPORT) {
-                    float *m = mo.maps + (long long)(3 * G.g) * mo.mplane + (long long)y * mo.mpitch + G.x0 + cc + j;
+                    float *m = ebuf + t_r * kExpRow + cc + j;
                     m[0] = d;
-                    m[mo.mplane] = art;
-                    m[2 * mo.mplane] = det;
+                    m[kExpMap] = art;
+                    m[2 * kExpMap] = det;
                 }
                 add_maps(ts, d, art, det);
             }
@@ -752,10 +774,10 @@ __device__ __forceinline__ void h_step(const float2 *__restrict__ buf, int r0, i
                     float d, art, det;
                     maps_px<true>(mA[j], mB[j], rw[j], kk, G.cg - kk, d, art, det);
                     if (EXPORT) {
-                        float *m = mo.maps + (long long)(3 * G.g) * mo.mplane + (long long)y * mo.mpitch + xx;
+                        float *m = ebuf + t_r * kExpRow + cc + j;
                         m[0] = d;
-                        m[mo.mplane] = art;
-                        m[2 * mo.mplane] = det;
+                        m[kExpMap] = art;
+                        m[2 * kExpMap] = det;
                     }
                     add_maps(ts, d, art, det);
                 }
@@ -881,6 +903,7 @@ __device__ __forceinline__ void flat_item(const Item<ST> &it, float2 *smb, float
     if (it.nsteps >= 2) issue_rows<ST>(it, 2, stage(2), &bars[0], warp, lane, withhold, ok);
     float2 *const buf = smb;
     double *sacc = (double *)(stages + kStages * kStageFloats) + tid;
+    float *const ebuf = (float *)(sacc - tid + 6 * kFusedThreads);  // EXPORT only
 #pragma unroll
     for (int m = 0; m < 6; m++) sacc[m * kFusedThreads] = 0.0;
     int next = 0;
@@ -894,8 +917,9 @@ __device__ __forceinline__ void flat_item(const Item<ST> &it, float2 *smb, float
         v_step<decltype(s0)::value>(R, in, cg, buf, tid);
         __syncthreads();
         if (st + 3 <= it.nsteps) issue_rows<ST>(it, st + 3, stage(st + 3), &bars[(st + 3) & 1], warp, lane, withhold, ok);
-        h_step<EXPORT>(buf, r, nr, t_r, t_s, t_on, G, sacc, mo);
+        h_step<EXPORT>(buf, r, nr, t_r, t_s, t_on, G, sacc, ebuf);
         __syncthreads();
+        if (EXPORT) export_rows(ebuf, r, nr, G, mo, tid);  // done before the next step's first barrier
     };
     for (int st = 0; st < it.nsteps; st += 2) {
         step(st, std::integral_constant<int, 0>());
@@ -911,7 +935,7 @@ __device__ __forceinline__ void flat_item(const Item<ST> &it, float2 *smb, float
     if (tid == 0) *s_next = next;
     if (!ok) *s_bad = 1;
     __syncthreads();
-    if (tid < 6) {
+    if (!EXPORT && tid < 6) {
         double v = 0.0;
 #pragma unroll
         for (int w = 0; w < kFusedThreads / 32; w++) v += s_warp[w][tid];
@@ -929,7 +953,7 @@ template <typename ST, bool EXPORT = false>
 __global__ void __launch_bounds__(kFusedThreads, kTileBlocks)
     fused_kernel(const DevPair *__restrict__ pairs, const Seg *__restrict__ segs, int nseg, int first_item,
                  int end_item, int *__restrict__ counter, TileCheck ck, double *__restrict__ partials,
-                 MapOut mo = MapOut{nullptr, 0, 0}) {
+                 MapOut mo) {
     extern __shared__ __align__(128) float2 smb[];  // [3 planes][kStep][kRS], then the stages and sums
     float *const stages = (float *)(smb + kBufF2);
     __shared__ int s_next, s_bad;
@@ -948,7 +972,7 @@ __global__ void __launch_bounds__(kFusedThreads, kTileBlocks)
     int item = first_item + blockIdx.x;  // the grid is at most the items
     while (item < end_item) {
         const int tile = item / 3, g = item - 3 * tile;
-        const Seg sg = segs[find_seg(segs, nseg, tile, tid & 31)];
+        const Seg sg = EXPORT ? mo.seg : segs[find_seg(segs, nseg, tile, tid & 31)];
         const Item<ST> it = decode_item<ST>(pairs[sg.pair], sg, tile, g);
         flat_item<ST, EXPORT>(it, smb, stages, s_bar, phase, ck, tid, s_warp, partials, item, mo, counter, &s_next,
                               &s_bad);
@@ -1093,6 +1117,8 @@ const double *host_weights() { return kWeights; }
 cudaError_t upload_weights() { return cudaMemcpyToSymbol(c_weight, kWeights, sizeof kWeights); }
 
 size_t fused_smem_bytes() { return (size_t)kBufF2 * sizeof(float2) + (size_t)kStages * kStageFloats * sizeof(float) + 6 * kFusedThreads * sizeof(double); }
+constexpr int kExportBlocks = kTileBlocks - 1;  // resident blocks per SM: the map rows take one block's room
+static size_t export_smem_bytes() { return fused_smem_bytes() + 3 * kExpMap * sizeof(float); }
 int fused_threads() { return kTileThreads; }
 
 template <bool EXPORT>
@@ -1102,7 +1128,8 @@ static cudaError_t fused_attrs() {
     // for the largest shared-memory carveout so that 4 blocks fit per SM
     cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
     if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fused_smem_bytes());
+    return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)(EXPORT ? export_smem_bytes() : fused_smem_bytes()));
 }
 
 cudaError_t configure_kernels() {
@@ -1179,19 +1206,15 @@ cudaError_t launch_fused(int storage, const DevPair *pairs, const Seg *segs, int
     grid = grid > nt ? nt : grid;
     (void)storage;
     return dep::launch(early, fused_kernel<float, false>, dim3(grid), kTileThreads, fused_smem_bytes(), st, pairs, segs, nseg,
-                        fi, ei, counter, ck, partials, MapOut{nullptr, 0, 0});
+                        fi, ei, counter, ck, partials, MapOut{});
 }
 
-cudaError_t launch_fused_export(int storage, const DevPair *pairs, const Seg *segs, int nseg, int first_tile,
-                                int end_tile, int *counter, const TileCheck &ck, double *partials, float *maps,
-                                long long mpitch, long long mplane, int grid, cudaStream_t st) {
-    const int fi = 3 * first_tile, ei = 3 * end_tile;
-    const int nt = ei - fi;
-    if (nt <= 0) return cudaSuccess;
-    grid = grid > nt ? nt : grid;
-    (void)storage;
-    fused_kernel<float, true><<<grid, kTileThreads, fused_smem_bytes(), st>>>(pairs, segs, nseg, fi, ei, counter,
-                                                                             ck, partials, MapOut{maps, mpitch, mplane});
+cudaError_t launch_fused_export(const DevPair *pairs, const Seg &seg, int ntiles, int *counter, const TileCheck &ck,
+                                float *maps, long long mpitch, long long mplane, int num_sms, cudaStream_t st) {
+    if (ntiles <= 0) return cudaSuccess;
+    const int items = 3 * ntiles, resident = num_sms * kExportBlocks;
+    fused_kernel<float, true><<<items < resident ? items : resident, kTileThreads, export_smem_bytes(), st>>>(
+        pairs, nullptr, 0, 0, items, counter, ck, nullptr, MapOut{maps, mpitch, mplane, seg});
     return cudaGetLastError();
 }
 
