@@ -182,3 +182,29 @@ def test_host_batch_with_dssim(tmb, cuda):
     got = b.results()
     assert [g[0] for g in got] == [w[0] for w in want]
     assert [g[5] for g in got] == [w[5] for w in want]
+
+
+@pytest.mark.parametrize("sizes", [[(8, 8), (9, 65), (119, 64), (120, 63), (121, 66)],
+                                   [(124, 129), (241, 70), (333, 211), (700, 14), (14, 700)],
+                                   [(500, 300), (1300, 701), (1921, 130)]])
+def test_strips_and_tiles_agree(tmb, cuda, sizes):
+    """A submission that fills the GPU runs DSSIM in strips, a small one in
+    tiles: each pair's values are the same bit for bit (widths around the strips'
+    120 columns, heights around their 64 rows, clamped levels)."""
+    g = cuda.Generator(device="cuda")
+    g.manual_seed(77)
+
+    def pair(w, h):
+        r = cuda.randint(0, 256, (h, w, 3), generator=g, device="cuda", dtype=cuda.uint8)
+        return tmb.PairDesc(r, (r // 8 * 8 + 4).to(cuda.uint8), "srgb8")
+
+    pairs = [pair(w, h) for w, h in sizes]
+    b = tmb.Ssim2Batch(8, 16 << 20)
+    b.set_metrics("dssim")
+    alone = [b.compute_batch([p])[0] for p in pairs]
+    big = pair(3840, 2160)  # more than two waves of strips
+    both = b.compute_batch(pairs[:2] + [big] + pairs[2:])
+    del both[2]
+    for a, c, s in zip(alone, both, sizes):
+        assert a[4] == c[4] == 0 and a[5] == c[5], s
+        assert np.array_equal(a[6], c[6]), s

@@ -11,6 +11,10 @@
 //                       channel-averaged SSIM (dssim-cuda-kernel/src/ssim.rs:
 //                       152-236), stored to the level's SSIM map, and the
 //                       tile's sum of SSIM in f64
+//   dssim_strip_kernel  the same map for submissions large enough to fill the
+//                       GPU with strips of 120 columns, walked row by row with
+//                       every stage in registers; dssim_sum_kernel then forms
+//                       the tiles' sums
 //   dssim_mean_kernel   per (pair, level): mean SSIM, avg = mean^(0.5^s)
 //                       (lib.rs:404-411)
 //   dssim_mad_kernel    per tile: sum of |avg - ssim| (ssim.rs:240-262)
@@ -34,7 +38,7 @@
 namespace s2 {
 
 // dssim-cuda-kernel/src/blur.rs:13-17
-__device__ __forceinline__ float ds_k(int i) {
+__host__ __device__ __forceinline__ float ds_k(int i) {
     return (i == 4) ? 0.146293f : ((i & 1) ? 0.118095f : 0.095332f);
 }
 
@@ -491,6 +495,412 @@ __global__ void __launch_bounds__(kDsThreads, kDsBlocks) dssim_tile_kernel(const
     }
 }
 
+// ---------------------------------------------------------------------------
+// strip pass
+// ---------------------------------------------------------------------------
+//
+// One block per strip of 120 columns x `rows` rows of a (pair, level), one
+// warp per Lab channel, walking down the rows with every blur stage's state
+// in registers: no stage is stored, and the next stage takes a row as soon as
+// it is formed.  Lane t holds four columns.
+//
+//   3x3 blur      out(row - 1) = top taps of row - 2, middle taps of row - 1,
+//                 bottom taps of row, added in the reference's row-major tap
+//                 order: each new row completes the output above it, extends
+//                 the output at it and starts the output below it (ds_step).
+//                 Two partial sums per column and plane are all a stage keeps,
+//                 and a row's products serve the three outputs.
+//   columns       a stage's four outputs are centred one column right of its
+//                 four inputs, so a lane needs only the first two inputs of the
+//                 lane after it (two shuffles) and its outer taps' products are
+//                 aligned f32x2 pairs.  Input column e of stage k of lane t is
+//                 X0 - 4 + 4 t + e + k (a, b: stages 0..3, the last output at
+//                 X0 + 4 t + e) or X0 - 2 + 4 t + e + k (L: two stages).  The
+//                 last lanes' outputs, which lack neighbours, fall in columns
+//                 >= 120, which the next strip owns.
+//   a, b warps    pre-blur, pre-blur, x^2 y^2 xy, two blurs of the five planes
+//                 (14 plane steps per row); per row they pass the six terms of
+//                 their pixels to the L warp through shared memory
+//   L warp        two blurs of five planes (10 plane steps), starting 4 rows
+//                 later; then (L + a) + b of the six terms and the SSIM
+//
+// What bounds it: FP32 instructions and their latency with three warps a
+// scheduler (112 registers of state): 38 plane steps per pixel, 16 f32x2 adds
+// and 20 multiplies per four outputs, where the tile pass below spends twice
+// that per output on windows that two threads form, shared-memory traffic and
+// 12 % of halo.  16 x 720p pairs (Lab of five levels): 727 us against the tile
+// pass's 962.  A strip is a chain of 40 to 136 dependent rows of about 2 us,
+// so a submission with few strips is faster in tiles (1600x1067: 140 against
+// 124 us): see choose_ds_rows.
+//
+namespace strip {
+
+struct DsRow {
+    float2 a, b;  // columns e = 0, 1 and 2, 3
+};
+
+// One plane's stage: the partial sums of the output at the last row (s2: top
+// and middle taps) and of the one below it (s1: top taps).
+struct DsStage {
+    float2 s1a, s1b, s2a, s2b;
+};
+
+__device__ __forceinline__ float2 ds_sum3(float2 s, float2 l, float2 m, float2 r) {
+    return __fadd2_rn(__fadd2_rn(__fadd2_rn(s, l), m), r);
+}
+
+// The corner and edge taps and -0 as pairs, from kernel arguments: the
+// compiler, which would build known constants anew for every use, keeps them.
+struct DsK {
+    float2 c, e, nz;
+};
+
+// An input row's products with the outer rows' taps (corner, edge, corner) for
+// the two output pairs: the left taps of the second are the right ones of the first.
+struct DsOuter {
+    float2 c0, c1, c2, e0, e1;
+};
+
+__device__ __forceinline__ DsOuter ds_outer(const DsRow &in, float2 n, const DsK &k) {
+    const float ke = ds_k(1);
+    return DsOuter{__ffma2_rn(k.c, in.a, k.nz), __ffma2_rn(k.c, in.b, k.nz), __ffma2_rn(k.c, n, k.nz),
+                   make_float2(ke * in.a.y, ke * in.b.x), make_float2(ke * in.b.y, ke * n.x)};
+}
+
+// the first two inputs of the next lane
+__device__ __forceinline__ float2 ds_next(const DsRow &in) {
+    return make_float2(__shfl_down_sync(0xffffffffu, in.a.x, 1), __shfl_down_sync(0xffffffffu, in.a.y, 1));
+}
+
+// The stage takes its next input row and gives the output centred one row up
+// and one column right.
+__device__ __forceinline__ DsRow ds_step(DsStage &S, const DsRow &in, const DsK &k) {
+    const float km = ds_k(4);
+    const float2 n = ds_next(in);
+    const DsOuter o = ds_outer(in, n, k);
+    DsRow out;
+    out.a = ds_sum3(S.s2a, o.c0, o.e0, o.c1);
+    out.b = ds_sum3(S.s2b, o.c1, o.e1, o.c2);
+    // middle row: edge, centre, edge
+    const float2 l0 = __ffma2_rn(k.e, in.a, k.nz), l1 = __ffma2_rn(k.e, in.b, k.nz), l2 = __ffma2_rn(k.e, n, k.nz);
+    S.s2a = ds_sum3(S.s1a, l0, make_float2(km * in.a.y, km * in.b.x), l1);
+    S.s2b = ds_sum3(S.s1b, l1, make_float2(km * in.b.y, km * n.x), l2);
+    S.s1a = __fadd2_rn(__fadd2_rn(o.c0, o.e0), o.c1);
+    S.s1b = __fadd2_rn(__fadd2_rn(o.c1, o.e1), o.c2);
+    return out;
+}
+
+// Before the stage takes row 0 of the level: the row above it repeats it.
+__device__ __forceinline__ void ds_top(DsStage &S, const DsRow &in, const DsK &k) {
+    const DsOuter o = ds_outer(in, ds_next(in), k);
+    S.s1a = __fadd2_rn(__fadd2_rn(o.c0, o.e0), o.c1);
+    S.s1b = __fadd2_rn(__fadd2_rn(o.c1, o.e1), o.c2);
+}
+
+constexpr int kStripW = kDsStripW;  // output columns of a strip
+constexpr int kStripThreads = 96;   // a warp each for L, a, b
+
+constexpr int kHoldPlanes = 9;  // 2 + 2 pre-blurred planes and 5 statistics
+
+// What an edge strip needs to replace the values of a stage outside the level
+// by those of the position clamped into it -- what the reference's next stage
+// reads there with clamped indexes.
+struct DsEdge {
+    int H;
+    bool cols, left;  // the strip's columns or their halo reach outside the level; on the left
+    int last;        // place of column W - 1 among the 128 columns of the outputs at X0 + 4 t + e
+    float4 *hold;    // this lane's slots for the stages' last rows
+};
+
+// An edge strip's stage output with `back` stages to go (its element e of
+// lane t is column X0 - back + 4 t + e): the columns outside the level, then,
+// from the row below the level on, the level's last row.  row: the output's
+// level row; slot: its plane's place in `hold`.
+__device__ __forceinline__ void ds_fix(DsRow &v, const DsEdge &E, int back, int row, int slot) {
+    float f[4] = {v.a.x, v.a.y, v.b.x, v.b.y};
+    const int lane = threadIdx.x & 31;
+    if (E.left && lane == 0) {
+#pragma unroll
+        for (int e = 0; e < 4; e++)
+            if (e < back) f[e] = f[back];
+    }
+    const int at = E.last + back;
+    if (at < 127) {
+        const int se = at & 3;
+        const float mine = se == 0 ? f[0] : (se == 1 ? f[1] : (se == 2 ? f[2] : f[3]));
+        const float last = __shfl_sync(0xffffffffu, mine, at >> 2);
+#pragma unroll
+        for (int e = 0; e < 4; e++)
+            if (4 * lane + e > at) f[e] = last;
+    }
+    float4 *h = E.hold + slot * 32;
+    if (row == E.H - 1) *h = make_float4(f[0], f[1], f[2], f[3]);
+    if (row >= E.H) {
+        const float4 t = *h;
+        f[0] = t.x, f[1] = t.y, f[2] = t.z, f[3] = t.w;
+    }
+    v.a = make_float2(f[0], f[1]);
+    v.b = make_float2(f[2], f[3]);
+}
+
+// SSIM of two pixels from the summed terms (ssim.rs:208-233)
+__device__ __forceinline__ float2 ds_ssim2(const float2 t[6], float2 nz) {
+    const float third = 1.0f / 3.0f;
+    const float2 th = make_float2(third, third), c1 = make_float2(0.0001f, 0.0001f), c2 = make_float2(0.0009f, 0.0009f);
+    const float2 two = make_float2(2.0f, 2.0f), neg = make_float2(-1.0f, -1.0f);
+    const float2 mu1_sq = __ffma2_rn(t[0], th, nz), mu2_sq = __ffma2_rn(t[1], th, nz);
+    const float2 mu1_mu2 = __ffma2_rn(t[2], th, nz);
+    // a - b as b * -1 + a: one rounding, that of the subtraction
+    const float2 sigma1_sq = __ffma2_rn(mu1_sq, neg, __ffma2_rn(t[3], th, nz));
+    const float2 sigma2_sq = __ffma2_rn(mu2_sq, neg, __ffma2_rn(t[4], th, nz));
+    const float2 sigma12 = __ffma2_rn(mu1_mu2, neg, __ffma2_rn(t[5], th, nz));
+    const float2 n1 = __ffma2_rn(two, mu1_mu2, c1), n2 = __ffma2_rn(two, sigma12, c2);
+    const float2 d1 = __fadd2_rn(__fadd2_rn(mu1_sq, mu2_sq), c1);
+    const float2 d2 = __fadd2_rn(__fadd2_rn(sigma1_sq, sigma2_sq), c2);
+    return make_float2((n1.x * n2.x) / (d1.x * d2.x), (n1.y * n2.y) / (d1.y * d2.y));
+}
+
+constexpr int kRawRows = 4;   // raw rows in flight: three ahead
+constexpr int kTermRows = 2;  // rows that a and b may be ahead of L
+
+// Named barriers of a terms slot: `full` (a and b arrive, L waits) and
+// `empty` (L arrives, a and b wait).  Every row of a and b from the third on
+// waits for the arrival L makes for the row kTermRows before it, and for no
+// other, so arrivals and waits pair up.
+__device__ __forceinline__ void ds_arrive(int id) {
+    asm volatile("barrier.cta.arrive %0, %1;" ::"r"(id), "n"(96) : "memory");
+}
+__device__ __forceinline__ void ds_wait(int id) {
+    asm volatile("barrier.cta.sync %0, %1;" ::"r"(id), "n"(96) : "memory");
+}
+
+struct DsShared {
+    float4 raw[3][kRawRows][2][32];   // [warp][row][image][lane]
+    float4 terms[kTermRows][2][6][32];  // [row][a, b][term][lane]
+    float4 hold[3][kHoldPlanes][32];  // [warp][plane][lane], edge strips only
+};
+
+// All three warps run this one loop (the statistics are the bulk of it and
+// the same for every channel: with a body per role, and one more per role for
+// edge strips, the SM's warps waited for instructions more than for anything
+// else, 1312 us where this takes 727).
+__device__ __forceinline__ void ds_strip(const DsPair &P, int level, int X0, int Y0, int rows,
+                                         const DsK &K, DsShared &sh) {
+    const float2 nz = K.nz;
+    const int W = P.w[level], H = P.h[level], pitch = P.pitch[level];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const bool ab = warp != 0;
+    const int yend = min(Y0 + rows, H);  // output rows [Y0, yend)
+    DsEdge E;
+    E.cols = X0 == 0 || X0 + 126 > W;  // L's last lane reads to X0 + 125
+    E.left = X0 == 0;
+    E.last = W - 1 - X0;
+    E.H = H;
+    E.hold = &sh.hold[warp][0][lane];
+    // raw input: columns X0 - 4 + 4 t + e of a and b, X0 - 2 + 4 t + e of L
+    const int x0 = X0 - (ab ? 4 : 2) + 4 * lane;
+    const int ca = ds_clamp(x0, W - 1), cb = ds_clamp(x0 + 1, W - 1), cc = ds_clamp(x0 + 2, W - 1),
+              cd = ds_clamp(x0 + 3, W - 1);
+    const long long plane = (long long)pitch * H;
+    const long long other = P.lab[1][level] - P.lab[0][level];
+    // a lane copies and reads its own columns only, so no warp waits for another's copies
+    float4 *const ring = &sh.raw[warp][0][0][lane];
+    // the raw row to fetch next, clamped into the level, and its samples
+    int fetch_row = Y0 - (ab ? 4 : 2);
+    const float *src = P.lab[0][level] + warp * plane + (long long)ds_clamp(fetch_row, H - 1) * pitch;
+    auto fetch = [&](int slot) {
+        float *d = (float *)(ring + slot * 64);
+        if (E.cols) {
+            const float *b = src;
+#pragma unroll
+            for (int img = 0; img < 2; img++) {
+                ds_cp<4>(d, b + ca);
+                ds_cp<4>(d + 1, b + cb);
+                ds_cp<4>(d + 2, b + cc);
+                ds_cp<4>(d + 3, b + cd);
+                b += other, d += 128;
+            }
+        } else {
+            const float *b = src + x0;
+            ds_cp<8>(d, b);
+            ds_cp<8>(d + 2, b + 2);
+            ds_cp<8>(d + 128, b + other);
+            ds_cp<8>(d + 130, b + other + 2);
+        }
+        if (fetch_row >= 0 && fetch_row < H - 1) src += pitch;
+        fetch_row++;
+    };
+    auto take = [&](int slot, int img) {
+        const float4 f = ring[slot * 64 + img * 32];
+        return DsRow{make_float2(f.x, f.y), make_float2(f.z, f.w)};
+    };
+    const DsStage zero{};
+    DsStage A1[2], A2[2], B1[5], B2[5];
+#pragma unroll
+    for (int p = 0; p < 2; p++) A1[p] = zero, A2[p] = zero;
+#pragma unroll
+    for (int p = 0; p < 5; p++) B1[p] = zero, B2[p] = zero;
+    // step i: the inputs of the statistics are row Y0 - 6 + i, for which a and
+    // b take their raw row Y0 - 4 + i; the output row is Y0 - 8 + i
+    const int n = yend - Y0 + 8;
+    int i = ab ? 0 : 4;  // L has no pre-blur to fill
+    for (int k = 0; k < kRawRows - 1; k++) {
+        fetch((i + k) % kRawRows);  // n >= 9: these rows are all wanted
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    }
+    float *map = P.map[level] + (long long)Y0 * pitch + X0 + 4 * lane;
+#pragma unroll 1
+    for (; i < n; i++) {
+        if (i + kRawRows - 1 < n) fetch((i + kRawRows - 1) % kRawRows);
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(kRawRows - 1) : "memory");
+        DsRow cx = take(i % kRawRows, 0), cy = take(i % kRawRows, 1);
+        const int row = Y0 - 6 + i;
+        // columns outside the level, or rows of this step's outputs (row + 1
+        // to row - 1) at its top or bottom, to be replaced
+        const bool fix = E.cols || row <= 1 || row + 2 >= H;
+        DsRow q[5];
+        if (ab) {
+            cx = ds_step(A1[0], cx, K);
+            cy = ds_step(A1[1], cy, K);
+            if (fix) {
+                ds_fix(cx, E, 3, row + 1, 0);
+                ds_fix(cy, E, 3, row + 1, 1);
+                if (row + 1 == 0) ds_top(A2[0], cx, K), ds_top(A2[1], cy, K);
+            }
+            cx = ds_step(A2[0], cx, K);
+            cy = ds_step(A2[1], cy, K);
+            if (fix) {
+                ds_fix(cx, E, 2, row, 2);
+                ds_fix(cy, E, 2, row, 3);
+            }
+            if (i < 4) continue;
+        }
+        q[0] = cx;
+        q[1] = cy;
+        q[2] = DsRow{__ffma2_rn(cx.a, cx.a, nz), __ffma2_rn(cx.b, cx.b, nz)};
+        q[3] = DsRow{__ffma2_rn(cy.a, cy.a, nz), __ffma2_rn(cy.b, cy.b, nz)};
+        q[4] = DsRow{__ffma2_rn(cx.a, cy.a, nz), __ffma2_rn(cx.b, cy.b, nz)};
+        if (fix && row == 0) {
+#pragma unroll
+            for (int p = 0; p < 5; p++) ds_top(B1[p], q[p], K);
+        }
+#pragma unroll
+        for (int p = 0; p < 5; p++) {
+            q[p] = ds_step(B1[p], q[p], K);
+            if (fix) {
+                ds_fix(q[p], E, 1, row - 1, 4 + p);
+                if (row - 1 == 0) ds_top(B2[p], q[p], K);
+            }
+            q[p] = ds_step(B2[p], q[p], K);
+        }
+        // the pixels' six terms: mu1^2, mu2^2, mu1 mu2, blur(x^2), blur(y^2), blur(xy)
+        DsRow t[6];
+        t[0] = DsRow{__ffma2_rn(q[0].a, q[0].a, nz), __ffma2_rn(q[0].b, q[0].b, nz)};
+        t[1] = DsRow{__ffma2_rn(q[1].a, q[1].a, nz), __ffma2_rn(q[1].b, q[1].b, nz)};
+        t[2] = DsRow{__ffma2_rn(q[0].a, q[1].a, nz), __ffma2_rn(q[0].b, q[1].b, nz)};
+        t[3] = q[2], t[4] = q[3], t[5] = q[4];
+        if (i < 8) continue;
+        const int slot = i % kTermRows;
+        if (ab) {
+            if (i >= 8 + kTermRows) ds_wait(1 + kTermRows + slot);
+#pragma unroll
+            for (int m = 0; m < 6; m++)
+                sh.terms[slot][warp - 1][m][lane] = make_float4(t[m].a.x, t[m].a.y, t[m].b.x, t[m].b.y);
+            ds_arrive(1 + slot);
+            continue;
+        }
+        ds_wait(1 + slot);
+        float2 ta[6], tb[6];
+#pragma unroll
+        for (int m = 0; m < 6; m++) {
+            const float4 u = sh.terms[slot][0][m][lane], v = sh.terms[slot][1][m][lane];
+            ta[m] = __fadd2_rn(__fadd2_rn(t[m].a, make_float2(u.x, u.y)), make_float2(v.x, v.y));
+            tb[m] = __fadd2_rn(__fadd2_rn(t[m].b, make_float2(u.z, u.w)), make_float2(v.z, v.w));
+        }
+        if (i + kTermRows < n) ds_arrive(1 + kTermRows + slot);
+        const float2 sa = ds_ssim2(ta, nz), sb = ds_ssim2(tb, nz);
+        const int left = W - (X0 + 4 * lane);  // columns of the level from this lane's first on
+        if (lane < kStripW / 4) {
+            if (left >= 4) {
+                *(float4 *)map = make_float4(sa.x, sa.y, sb.x, sb.y);
+            } else if (left > 0) {
+                map[0] = sa.x;
+                if (left > 1) map[1] = sa.y;
+                if (left > 2) map[2] = sb.x;
+            }
+        }
+        map += pitch;
+    }
+}
+
+static_assert(kDsStripBlocks == 4, "168 registers, 38 KB shared per block");
+
+__global__ void __launch_bounds__(kStripThreads, kDsStripBlocks) dssim_strip_kernel(const DsPair *__restrict__ pairs,
+                                                                               const DsSeg *__restrict__ segs,
+                                                                               int nseg, int rows, float4 taps) {
+    __shared__ DsShared sh;
+    // -0 too is an argument: the compiler cannot turn the FMAs with it into multiplies
+    const DsK K{make_float2(taps.x, taps.x), make_float2(taps.y, taps.y), make_float2(taps.z, taps.z)};
+    int lo = 0, hi = nseg - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (segs[mid].first_strip <= (int)blockIdx.x) lo = mid;
+        else hi = mid - 1;
+    }
+    const DsSeg sg = segs[lo];
+    const DsPair &P = pairs[sg.pair];
+    const int local = blockIdx.x - sg.first_strip, sx = ds_strips_x(P.w[sg.level]);
+    const int X0 = local % sx * kStripW, Y0 = local / sx * rows;
+    ds_strip(P, sg.level, X0, Y0, rows, K, sh);
+}
+
+// The strips' map summed per 32 x 32 tile, in the tile pass's order to the
+// last addition (a pair's DSSIM is the same whichever of the two ran): there
+// thread t sums the 2 x 2 outputs at columns 2 (t % 16), rows 2 (t / 16), a
+// warp its lanes by a shuffle tree, and the block its 8 warps in order.  Here one
+// warp takes a tile, all 8 warps' values in flight at once (a block per tile,
+// with its two barriers, took 42 us for 16 x 720p pairs, this 33).
+__global__ void __launch_bounds__(kDsThreads) dssim_sum_kernel(const DsPair *__restrict__ pairs,
+                                                               const DsSeg *__restrict__ segs, int nseg, int ntiles,
+                                                               double *__restrict__ partials) {
+    constexpr int kWarps = kDsThreads / 32;
+    static_assert(kDsOutCols == 16 && kDsOutRows == 2, "half a warp per two rows");
+    dep::grid_wait();
+    const int tile = blockIdx.x * kWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (tile >= ntiles) return;
+    const DsSeg sg = segs[ds_find_seg(segs, nseg, tile)];
+    const DsPair &P = pairs[sg.pair];
+    const int W = P.w[sg.level], H = P.h[sg.level], tl = tile - sg.first_tile;
+    const int ox = tl % sg.tiles_x * kDsT + 2 * (lane % 16), oy = tl / sg.tiles_x * kDsT + 2 * (lane / 16);
+    const long long pitch = P.pitch[sg.level];
+    const float *map = P.map[sg.level] + (long long)oy * pitch + ox;  // ox even: 8-byte aligned pairs
+    double v[kWarps];
+    const bool c0 = ox < W, c1 = ox + 1 < W;
+#pragma unroll
+    for (int w = 0; w < kWarps; w++) {
+        double sum = 0.0;
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            const bool in = oy + 4 * w + r < H;
+            const float2 f = in && c0 ? *(const float2 *)(map + (4 * w + r) * pitch) : make_float2(0.0f, 0.0f);
+            if (in && c0) sum += (double)f.x;
+            if (in && c1) sum += (double)f.y;
+        }
+        v[w] = sum;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int w = 0; w < kWarps; w++) v[w] += __shfl_down_sync(0xffffffffu, v[w], o);
+    double sum = 0.0;
+#pragma unroll
+    for (int w = 0; w < kWarps; w++) sum += v[w];
+    if (lane == 0) partials[tile] = sum;
+}
+
+}  // namespace strip
+
 // per (pair, level): mean SSIM and avg = max(mean, 0)^(0.5^s) as f32
 // (lib.rs:404-411; the reference casts avg to f32 for the |avg - ssim| pass)
 __global__ void __launch_bounds__(kDsThreads) dssim_mean_kernel(const DsPair *__restrict__ pairs,
@@ -594,8 +1004,8 @@ cudaError_t configure_dssim_kernels() {
                                 (int)(kDsSmemFloats * sizeof(float)));
 }
 
-cudaError_t launch_dssim(const DsPair *pairs, int npairs, const DsSeg *segs, int nseg, int ntiles, bool clamp,
-                         double *partials, float *avg, DevResult *out, bool write_all, int num_sms,
+cudaError_t launch_dssim(const DsPair *pairs, int npairs, const DsSeg *segs, int nseg, int ntiles, int nstrips,
+                         int strip_rows, bool clamp, double *partials, float *avg, DevResult *out, bool write_all, int num_sms,
                          cudaStream_t st) {
     if (npairs <= 0) return cudaSuccess;
     // the small passes behind the tile pass launch dependently (1600x1067, one
@@ -606,8 +1016,16 @@ cudaError_t launch_dssim(const DsPair *pairs, int npairs, const DsSeg *segs, int
         // persistent: the resident blocks of the tile kernel (4 per SM), each
         // striding over the tiles
         const int grid = ntiles < num_sms * kDsBlocks ? ntiles : num_sms * kDsBlocks;
-        e = dep::launch(false, dssim_tile_kernel, dim3(grid), kDsThreads, kDsSmemFloats * sizeof(float), st, pairs, segs,
-                        nseg, ntiles, partials, -0.0f);
+        if (strip_rows) {
+            e = dep::launch(false, strip::dssim_strip_kernel, dim3(nstrips), strip::kStripThreads, 0, st, pairs, segs,
+                            nseg, strip_rows, make_float4(ds_k(0), ds_k(1), -0.0f, 0.0f));
+            if (e != cudaSuccess) return e;
+            e = dep::launch(true, strip::dssim_sum_kernel, dim3((ntiles + kMadWarps - 1) / kMadWarps), kDsThreads, 0, st,
+                            pairs, segs, nseg, ntiles, partials);
+        } else {
+            e = dep::launch(false, dssim_tile_kernel, dim3(grid), kDsThreads, kDsSmemFloats * sizeof(float), st, pairs,
+                            segs, nseg, ntiles, partials, -0.0f);
+        }
         if (e != cudaSuccess) return e;
         e = dep::launch(true, dssim_mean_kernel, dim3(npairs * kDsLevels), kDsThreads, 0, st, pairs, partials, avg);
         if (e != cudaSuccess) return e;

@@ -87,13 +87,18 @@ struct DsPair {
     int status;
 };
 
-// A run of DSSIM tiles (32 x 32 outputs) of one (pair, level).
+// A run of DSSIM tiles (32 x 32 outputs), and of strips when the submission
+// runs in them, of one (pair, level).
 struct DsSeg {
     int first_tile;
     int pair;
     int level;
     int tiles_x;
+    int first_strip;
 };
+constexpr int kDsStripW = 120;     // output columns of a strip
+constexpr int kDsStripBlocks = 4;  // resident strips per SM
+__host__ __device__ __forceinline__ int ds_strips_x(int w) { return (w + kDsStripW - 1) / kDsStripW; }
 
 // A run of tiles of one (pair, scale); tiles are numbered across segments.
 struct Seg {

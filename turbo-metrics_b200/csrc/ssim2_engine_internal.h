@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <string>
 #include <vector>
@@ -148,6 +149,7 @@ struct Plan {
     std::vector<DsPair> ds;
     std::vector<DsSeg> dsegs;
     int ds_tiles = 0;
+    int ds_strips = 0, ds_rows = 0;  // strips of ds_rows rows, or 0: the tile pass
     bool ds_clamp = false;
 
     // descriptor region: pairs | blk_first | segs | IIR vsegs | hsegs | DSSIM pairs | DSSIM segs
@@ -460,6 +462,29 @@ struct Engine {
         return blocks <= 2 * (uint64_t)num_sms ? kPyrBlkSmall : kPyrBlk;
     }
 
+    // DSSIM's map in strips (returns their rows) or in tiles (0).  A strip is
+    // a chain of rows, 8 more than it gives, so a submission needs a few waves
+    // of resident strips before their lower work per pixel shows; then the
+    // height with the least rows in all, in whole waves.  Tiles against strips:
+    // 1920x1080 DSSIM (0.6 waves of 64 rows) 234 / 273 us a call, 3840x2160 (2.5)
+    // 691 / 596, 16 x 720p (4.9) tile pass 962 against 727 + 30 for the sums.
+    int choose_ds_rows(const Plan &P) const {
+        const double resident = (double)kDsStripBlocks * num_sms;
+        double best = 0.0;
+        int best_rows = 0;
+        for (int rows : {64, 128}) {
+            double strips = 0;
+            for (const DsPair &D : P.ds)
+                if (D.status == 0)
+                    for (int s = 0; s < kDsLevels; s++)
+                        strips += (double)ds_strips_x(D.w[s]) * ((D.h[s] + rows - 1) / rows);
+            if (strips < 2 * resident) continue;
+            const double cost = (rows + 8) * std::ceil(strips / resident);
+            if (!best_rows || cost < best) best = cost, best_rows = rows;
+        }
+        return best_rows;
+    }
+
     // Lay out the levels and tiles of n pairs.
     s2_status plan(const s2_pair_desc *d, int n, Plan &P, const PairExtra *ex = nullptr, int ngroups = 1) {
         P = Plan();
@@ -557,6 +582,7 @@ struct Engine {
                 if (P.pairs[i].status != S2_OK) P.ds[i].status = P.pairs[i].status;
             // DSSIM tiles: all pairs' level 0 first, then level 1, ...
             int dt = 0;
+            P.ds_rows = choose_ds_rows(P);
             for (int s = 0; s < kDsLevels; s++)
                 for (int i = 0; i < n; i++) {
                     DsPair &D = P.ds[i];
@@ -569,6 +595,8 @@ struct Engine {
                     D.tile_base[s] = dt;
                     D.tile_cnt[s] = sg.tiles_x * ((D.h[s] + 31) / 32);
                     dt += D.tile_cnt[s];
+                    sg.first_strip = P.ds_strips;
+                    if (P.ds_rows) P.ds_strips += ds_strips_x(D.w[s]) * ((D.h[s] + P.ds_rows - 1) / P.ds_rows);
                     P.dsegs.push_back(sg);
                 }
             P.ds_tiles = dt;
@@ -785,9 +813,9 @@ struct Engine {
         const int pout = (m_s2 ? 1 : 0) | (m_ds ? 2 : 0);
         if (graphs && !host && !profiling && ng == 1) {
             const uint64_t key[8] = {(uint64_t)n | ((uint64_t)(uniform_fmt(P) + 1) << 40),
-                                     (uint64_t)P.total_blocks | ((uint64_t)P.pyr_blk << 40),
+                                     (uint64_t)P.total_blocks | ((uint64_t)P.pyr_blk << 40) | ((uint64_t)P.ds_rows << 52),
                                      (uint64_t)P.total_tiles,
-                                     P.segs.size(),
+                                     (uint64_t)P.segs.size() | ((uint64_t)(uint32_t)P.ds_strips << 32),
                                      P.vsegs.size(), P.hsegs.size(),
                                      ((uint64_t)(uint32_t)P.vtotal << 32) | (uint32_t)P.htotal,
                                      ((uint64_t)(uint32_t)P.ds_tiles << 32) | ((uint64_t)P.dsegs.size() << 3) |
@@ -896,7 +924,7 @@ struct Engine {
         double *part = (double *)ds_d.p;
         float *avg = (float *)((char *)ds_d.p + s2_align_up((size_t)2 * std::max(P.ds_tiles, 1) * sizeof(double), 256));
         return launch_dssim((const DsPair *)(dbase + L.ds_pairs()), n, (const DsSeg *)(dbase + L.ds_segs()),
-                            (int)P.dsegs.size(), P.ds_tiles, P.ds_clamp, part, avg, results_at(n),
+                            (int)P.dsegs.size(), P.ds_tiles, P.ds_strips, P.ds_rows, P.ds_clamp, part, avg, results_at(n),
                             (P.metrics & S2_METRIC_SSIMULACRA2) == 0, num_sms, st);
     }
 
