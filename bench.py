@@ -411,7 +411,7 @@ def dssim_bench(tmb, descs, n_pairs, steps, warmup, s2_value, peak):
     """DSSIM, the sibling metric, on the same batch: both metrics from one
     prep pass, and DSSIM alone; device-timed like the main leg, with the
     DSSIM passes' kernel time and their declared I/O (Lab planes of both
-    images read, SSIM map written by the tile pass and read by the MAD pass:
+    images read, SSIM map written once and read by the MAD pass:
     32 bytes per pixel over the five levels)."""
     import torch
     b = tmb.Ssim2Batch(n_pairs, n_pairs * W * H)
@@ -453,8 +453,8 @@ def dssim_bench(tmb, descs, n_pairs, steps, warmup, s2_value, peak):
         traffic = None
     out["roofline"] = {"bound": "hbm", "achieved": ab / (acc[3] / 1e3) / 1e9, "peak": peak, "unit": "GB/s",
                        "frac": ab / (acc[3] / 1e3) / 1e9 / peak, "algorithmic_bytes_per_launch": ab,
-                       "kernel": "dssim clamp+tile+mean+mad+final",
-                       # ncu DRAM bytes of the tile launch (the passes' dominant kernel), per launch
+                       "kernel": "dssim clamp+strip+sum+mean+mad+final",
+                       # ncu DRAM bytes of the map launch (strips at this size; the passes' dominant kernel)
                        "traffic_tile_kernel": traffic}
     out["both_vs_ssimulacra2_only"] = out["both_pairs_per_s"] / s2_value
     b.close()
