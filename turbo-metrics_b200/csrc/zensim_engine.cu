@@ -73,7 +73,24 @@ struct s2_zensim {
 
 static bool g_zs_lut_ready[64];
 
+// Bytes of saved sums up to which every channel of every scale has its own.
+// They add a quarter to the planes' memory, 34 GB at 65536 x 65536, where the
+// planes alone take 137; above this the channels take turns in those of one
+// channel of scale 0 (a sixteenth).  The line is at 2^30 pixels, where a
+// channel's walk has blocks for every SM (16384 columns: 512) and the turns
+// cost little; an image below it is short of blocks, not of memory.
+constexpr size_t kZsMaxState = (size_t)8 << 30;
+
+// s2_zensim_create with that limit given (0: the channels always take turns)
+extern "C" s2_status s2_zensim_create_limited(int32_t device, uint32_t width, uint32_t height, size_t max_state,
+                                              s2_zensim **out);
+
 s2_status s2_zensim_create(int32_t device, uint32_t width, uint32_t height, s2_zensim **out) {
+    return s2_zensim_create_limited(device, width, height, kZsMaxState, out);
+}
+
+s2_status s2_zensim_create_limited(int32_t device, uint32_t width, uint32_t height, size_t max_state,
+                                   s2_zensim **out) {
     if (!out) return S2_ERR_INVALID_ARG;
     *out = nullptr;
     // zensim-cuda/src/lib.rs:200-205
@@ -93,7 +110,7 @@ s2_status s2_zensim_create(int32_t device, uint32_t width, uint32_t height, s2_z
     // scales while the logical width and the height are >= 8 (lib.rs:222-233)
     ZsPlan &P = z->plan;
     int lw = (int)width, n = simd_padded_width((int)width), h = (int)height;
-    size_t bytes = 0, off[kZsScales][2], state[kZsScales];
+    size_t bytes = 0, states = 0, off[kZsScales][2], state[kZsScales];
     for (int s = 0; s < kZsScales; s++) {
         if (lw < 8 || h < 8) break;
         ZsScale &S = P.sc[s];
@@ -104,8 +121,8 @@ s2_status s2_zensim_create(int32_t device, uint32_t width, uint32_t height, s2_z
             off[s][img] = bytes;
             bytes += 3 * align_up(S.ref.pitch * h * sizeof(float), 256);
         }
-        state[s] = bytes;
-        bytes += align_up((size_t)3 * ((h + kZsSub - 1) / kZsSub) * 4 * S.ref.pitch * sizeof(float), 256);
+        state[s] = states;
+        states += align_up((size_t)3 * ((h + kZsSub - 1) / kZsSub) * 4 * S.ref.pitch * sizeof(float), 256);
         S.walk_x = (n + kZsWalkW - 1) / kZsWalkW;
         S.walk_first = P.walk_blocks;
         P.walk_blocks += 3 * S.walk_x;
@@ -118,7 +135,11 @@ s2_status s2_zensim_create(int32_t device, uint32_t width, uint32_t height, s2_z
         n = n / 2;
         h = (h + 1) / 2;
     }
-    z->plane_bytes = bytes;
+    const size_t planes = bytes;
+    P.one_channel = states > max_state;
+    if (P.one_channel)
+        states = align_up((size_t)((P.sc[0].h + kZsSub - 1) / kZsSub) * 4 * P.sc[0].ref.pitch * sizeof(float), 256);
+    z->plane_bytes = bytes += states;
     cudaError_t e = cudaMalloc(&z->planes, bytes);
     if (e == cudaSuccess) e = cudaMalloc((void **)&z->stage, (size_t)width * 3 * height);
     if (e == cudaSuccess)
@@ -133,7 +154,7 @@ s2_status s2_zensim_create(int32_t device, uint32_t width, uint32_t height, s2_z
         ZsPlanes *pl[2] = {&S.ref, &S.dis};
         for (int img = 0; img < 2; img++)
             for (int c = 0; c < 3; c++) pl[img]->p[c] = (float *)((char *)z->planes + off[s][img] + c * plane) + kZsLeft;
-        S.state = (float *)((char *)z->planes + state[s]);
+        S.state = (float *)((char *)z->planes + planes + (P.one_channel ? 0 : state[s]));
     }
     *out = z;
     return S2_OK;

@@ -496,9 +496,28 @@ cudaError_t zs_launch_prep(const uint8_t *img, size_t pitch, int w, int h, const
 }
 
 cudaError_t zs_launch_features(const ZsPlan &plan, double *tile_out, double *out, cudaStream_t st) {
-    cudaError_t e = dep::launch(true, zs_walk_kernel, dim3(plan.walk_blocks), kWalkThreads, kWalkSmem, st, plan);
-    if (e == cudaSuccess)
-        e = dep::launch(true, zs_feat_kernel, dim3(plan.tiles), kFeatThreads, kFeatSmem, st, plan, tile_out);
+    cudaError_t e = cudaSuccess;
+    const int parts = plan.one_channel ? 3 * plan.ns : 1;
+    for (int i = 0; i < parts && e == cudaSuccess; i++) {
+        ZsPlan part = plan;
+        double *part_out = tile_out;
+        if (plan.one_channel) {
+            // one channel of one scale as a plan of its own; its walk waits for
+            // the features that read the states before it
+            const int c = i % 3;
+            ZsScale &S = part.sc[0] = plan.sc[i / 3];
+            S.ref.p[0] = S.ref.p[c];
+            S.dis.p[0] = S.dis.p[c];
+            part.ns = 1;
+            part.walk_blocks = S.walk_x;
+            part.tiles = S.tiles_x * S.tiles_y;
+            part_out += (size_t)kZsOut * (S.tile_first + c * part.tiles);
+            S.walk_first = S.tile_first = 0;
+        }
+        e = dep::launch(true, zs_walk_kernel, dim3(part.walk_blocks), kWalkThreads, kWalkSmem, st, part);
+        if (e == cudaSuccess)
+            e = dep::launch(true, zs_feat_kernel, dim3(part.tiles), kFeatThreads, kFeatSmem, st, part, part_out);
+    }
     if (e == cudaSuccess)
         e = dep::launch(true, zs_reduce_kernel, dim3(plan.ns * 3), kZsOut * kRuns, 0, st, plan, tile_out, out);
     return e;

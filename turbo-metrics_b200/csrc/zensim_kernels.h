@@ -42,6 +42,7 @@ struct ZsPlan {
     ZsScale sc[kZsScales];
     int ns;
     int walk_blocks, tiles;
+    bool one_channel;  // the scales' channels share one channel's states (scale 0's): a walk and a feature launch each
 };
 
 cudaError_t zs_configure();
