@@ -97,6 +97,7 @@ struct DsSeg {
     int first_strip;
 };
 constexpr int kDsStripW = 120;     // output columns of a strip
+constexpr int kDsStripRows = 64;   // output rows of a strip
 constexpr int kDsStripBlocks = 4;  // resident strips per SM
 __host__ __device__ __forceinline__ int ds_strips_x(int w) { return (w + kDsStripW - 1) / kDsStripW; }
 

@@ -5,7 +5,6 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <cmath>
 #include <cstring>
 #include <string>
 #include <vector>
@@ -462,27 +461,42 @@ struct Engine {
         return blocks <= 2 * (uint64_t)num_sms ? kPyrBlkSmall : kPyrBlk;
     }
 
-    // DSSIM's map in strips (returns their rows) or in tiles (0).  A strip is
-    // a chain of rows, 8 more than it gives, so a submission needs a few waves
-    // of resident strips before their lower work per pixel shows; then the
-    // height with the least rows in all, in whole waves.  Tiles against strips:
-    // 1920x1080 DSSIM (0.6 waves of 64 rows) 234 / 273 us a call, 3840x2160 (2.5)
-    // 691 / 596, 16 x 720p (4.9) tile pass 962 against 727 + 30 for the sums.
+    // DSSIM's map in strips (returns their rows) or in tiles (0), by what each
+    // would take: per resident block, the time of a strip's row steps (8 more
+    // than its rows; one at the level's left or right edge also replaces the
+    // columns outside, whatever part of its 120 columns the level fills) and of
+    // a tile (one at an edge fixes up every stage).  The four rates and the fixed
+    // difference are a least-squares fit to the DSSIM passes of 50 submissions
+    // from 300 8x8 pairs to one 7680x4320 (B200, 148 SMs); a submission goes in
+    // strips where that predicts 3 % less.  Tiles / strips, us: 256 64x64 187 /
+    // 265, 64 256x256 369 / 399, 64 130x600 616 / 684, 64 121x512 407 / 594
+    // (narrow levels leave most columns of a strip empty), 32 512x512 627 / 577,
+    // 16 1280x720 979 / 768, 3840x2160 497 / 430, 64 1920x1080 8230 / 5377; 20
+    // more sizes bear the rule out but for 80 245x130 (339 / 385).  Below two
+    // waves of strips the fit is no guide (a strip is a chain of 72 rows:
+    // 4 1280x720 260 / 278, 1920x1080 161 / 192): tiles.  128-row strips took 1 to
+    // 5 % less at 16 3840x2160 and 64 2000x96, and 5 to 20 % more at 3 3840x2160, 8
+    // 1920x1080 and smaller submissions: not offered.
     int choose_ds_rows(const Plan &P) const {
+        const double row_inner = 1.85, row_edge = 2.45, tile_inner = 24.4, tile_edge = 44.3, fixed = 57.0;
         const double resident = (double)kDsStripBlocks * num_sms;
-        double best = 0.0;
-        int best_rows = 0;
-        for (int rows : {64, 128}) {
-            double strips = 0;
-            for (const DsPair &D : P.ds)
-                if (D.status == 0)
-                    for (int s = 0; s < kDsLevels; s++)
-                        strips += (double)ds_strips_x(D.w[s]) * ((D.h[s] + rows - 1) / rows);
-            if (strips < 2 * resident) continue;
-            const double cost = (rows + 8) * std::ceil(strips / resident);
-            if (!best_rows || cost < best) best = cost, best_rows = rows;
+        double strips = 0.0, strip_us = 0.0, tile_us = 0.0;
+        for (const DsPair &D : P.ds) {
+            if (D.status != 0) continue;
+            for (int s = 0; s < kDsLevels; s++) {
+                const int W = D.w[s], H = D.h[s];
+                const int sx = ds_strips_x(W), inner = std::max(W - 6, kDsStripW) / kDsStripW - 1;
+                const double steps = (double)(H / kDsStripRows) * (kDsStripRows + 8) +
+                                     (H % kDsStripRows ? H % kDsStripRows + 8 : 0);
+                strips += (double)sx * ((H + kDsStripRows - 1) / kDsStripRows);
+                strip_us += steps * (inner * row_inner + (sx - inner) * row_edge);
+                const double all = (double)((W + 31) / 32) * ((H + 31) / 32);
+                const double in = (double)(std::max(W - 4, 32) / 32 - 1) * (std::max(H - 4, 32) / 32 - 1);
+                tile_us += in * tile_inner + (all - in) * tile_edge;
+            }
         }
-        return best_rows;
+        if (strips < 2 * resident) return 0;
+        return fixed * resident + strip_us < 0.97 * tile_us ? kDsStripRows : 0;
     }
 
     // Lay out the levels and tiles of n pairs.
