@@ -495,6 +495,10 @@ s2_status s2_batch_last_dssim_ms(s2_batch *b, float *ms);
  * withholds nothing.  Process-wide; read when a submission is enqueued (a
  * CUDA graph keeps the values it was captured with). */
 s2_status s2_debug_tile_timeout(int32_t drop_item, int64_t wait_cycles);
+/* The form of the DSSIM map pass for later submissions of the batch: 64 strips
+ * of 64 rows, 0 tiles of 32 x 32, -1 (the default) the one that the engine
+ * expects to be faster.  Both give the same bits; for the tests and for timing. */
+s2_status s2_debug_dssim_rows(s2_batch *b, int32_t rows);
 /* Resident blocks per SM of the fused kernel for a storage type (0 on error). */
 int32_t s2_fused_blocks_per_sm(int32_t storage);
 

@@ -191,6 +191,7 @@ _sig = {
     "s2_batch_last_timings": (ctypes.c_int, [P, ctypes.POINTER(ctypes.c_float)]),
     "s2_fused_blocks_per_sm": (ctypes.c_int32, [ctypes.c_int32]),
     "s2_debug_tile_timeout": (ctypes.c_int, [ctypes.c_int32, ctypes.c_int64]),
+    "s2_debug_dssim_rows": (ctypes.c_int, [P, ctypes.c_int32]),
     "s2_server_config_default": (None, [ctypes.POINTER(ServerConfig)]),
     "s2_server_create": (ctypes.c_int, [ctypes.POINTER(ServerConfig), ctypes.POINTER(P)]),
     "s2_server_destroy": (None, [P]),

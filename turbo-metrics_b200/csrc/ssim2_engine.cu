@@ -295,6 +295,7 @@ struct s2_batch {
     int last_slot = 0;
     bool profiling = false, graphs = true;
     int metrics = S2_METRIC_SSIMULACRA2;
+    int ds_rows = -1;  // s2_debug_dssim_rows
     s2_config cfg;
     uint32_t max_pairs = 0;
     uint64_t max_pixels = 0;
@@ -315,6 +316,7 @@ struct s2_batch {
         }
         eng[k].graphs = graphs;
         eng[k].metrics = metrics;
+        eng[k].ds_rows_cfg = ds_rows;
         ready[k] = true;
         return S2_OK;
     }
@@ -1004,6 +1006,14 @@ s2_status s2_batch_set_metrics(s2_batch *b, int32_t metrics) {
     b->metrics = metrics;
     for (int k = 0; k < 2; k++)
         if (b->ready[k]) b->eng[k].metrics = metrics;
+    return S2_OK;
+}
+
+s2_status s2_debug_dssim_rows(s2_batch *b, int32_t rows) {
+    if (!b || (rows != -1 && rows != 0 && rows != kDsStripRows)) return S2_ERR_INVALID_ARG;
+    b->ds_rows = rows;
+    for (int k = 0; k < 2; k++)
+        if (b->ready[k]) b->eng[k].ds_rows_cfg = rows;
     return S2_OK;
 }
 

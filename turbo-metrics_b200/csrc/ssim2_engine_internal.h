@@ -370,6 +370,7 @@ struct Engine {
     }
 
     int force_strip = 0;  // a tuning trial's tile height (0 = none)
+    int ds_rows_cfg = -1;  // DSSIM's strip rows, 0 for tiles, -1 by choose_ds_rows (s2_debug_dssim_rows)
 
     // The fused pass's tile height (rows per strip): configured (16/32/64), a
     // tuning trial's, the autotuner's measured choice for this workload class,
@@ -478,6 +479,7 @@ struct Engine {
     // 5 % less at 16 3840x2160 and 64 2000x96, and 5 to 20 % more at 3 3840x2160, 8
     // 1920x1080 and smaller submissions: not offered.
     int choose_ds_rows(const Plan &P) const {
+        if (ds_rows_cfg >= 0) return ds_rows_cfg;
         const double row_inner = 1.85, row_edge = 2.45, tile_inner = 24.4, tile_edge = 44.3, fixed = 57.0;
         const double resident = (double)kDsStripBlocks * num_sms;
         double strips = 0.0, strip_us = 0.0, tile_us = 0.0;
