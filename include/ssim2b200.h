@@ -451,6 +451,12 @@ s2_status s2_compute_srgb8_noalloc(const uint8_t *ref, size_t ref_pitch, const u
 typedef struct s2_zensim s2_zensim;
 /* Replaces Zensim::new (lib.rs:198-287): S2_ERR_INVALID_SIZE below 8x8. */
 s2_status s2_zensim_create(int32_t device, uint32_t width, uint32_t height, s2_zensim **out);
+/* The same with a limit on the bytes of saved vertical sums (s2_zensim_create:
+ * 8 GiB).  Above it, and where the device has no room for more, the channels
+ * take turns in the sums of one channel (0: always): a sixteenth of the memory, a
+ * launch pair per channel, the same features to the bit. */
+s2_status s2_zensim_create_limited(int32_t device, uint32_t width, uint32_t height, size_t max_state,
+                                   s2_zensim **out);
 void s2_zensim_destroy(s2_zensim *z);
 /* Replaces Zensim::set_reference (lib.rs:340-376): packed sRGB8 rows of
  * `pitch` bytes, on the device or (on_host) in host memory; the reference's

@@ -58,10 +58,11 @@ struct s2_zensim {
     int device = 0;
     uint32_t w = 0, h = 0;
     ZsPlan plan = {};
-    void *planes = nullptr;       // both pyramids, then the saved states of the vertical sums
+    void *planes = nullptr;       // both pyramids, then the work area unless it lies in `stage`
     size_t plane_bytes = 0;
     uint8_t *stage = nullptr;     // device copy of host inputs (w * 3 * h bytes)
-    double *tile_out = nullptr;   // kZsOut doubles per tile, then per (scale, channel)
+    size_t stage_bytes() const { return (size_t)w * 3 * h; }
+    double *tile_out = nullptr;   // work area: kZsOut doubles per tile, then per (scale, channel)
     double out_h[kZsScales * 3 * kZsOut];  // host copy of the latter
     bool has_ref = false;
     double raw_acc[kZsScales][3][kZsSums];
@@ -75,15 +76,41 @@ static bool g_zs_lut_ready[64];
 
 // Bytes of saved sums up to which every channel of every scale has its own.
 // They add a quarter to the planes' memory, 34 GB at 65536 x 65536, where the
-// planes alone take 137; above this the channels take turns in those of one
-// channel of scale 0 (a sixteenth).  The line is at 2^30 pixels, where a
-// channel's walk has blocks for every SM (16384 columns: 512) and the turns
-// cost little; an image below it is short of blocks, not of memory.
+// planes alone take 137; above this, and where the device has no room for them,
+// the channels take turns in those of one channel of scale 0 (a sixteenth).
+// The line is at 2^30 pixels, where a channel's walk has blocks for every SM
+// (16384 columns: 512) and the turns cost little; an image below it is short of
+// blocks, not of memory.
 constexpr size_t kZsMaxState = (size_t)8 << 30;
 
-// s2_zensim_create with that limit given (0: the channels always take turns)
-extern "C" s2_status s2_zensim_create_limited(int32_t device, uint32_t width, uint32_t height, size_t max_state,
-                                              s2_zensim **out);
+// The device buffers of z, the saved sums by channels in turns (one_channel)
+// or all beside each other (states bytes, the first `state` of each scale).
+// What the features need besides the planes -- the saved sums and the tiles'
+// records -- follows the planes, or, in turns, lies in the host inputs' copy
+// where that is large enough (2.4 of its 3 bytes per pixel): the copy is read by
+// the prep pass and free afterwards, so an image then needs no more memory
+// than its planes and inputs.
+static cudaError_t zs_allocate(s2_zensim *z, size_t planes, size_t states, const size_t *state, bool one_channel) {
+    ZsPlan &P = z->plan;
+    P.one_channel = one_channel;
+    if (one_channel)
+        states = align_up((size_t)((P.sc[0].h + kZsSub - 1) / kZsSub) * 4 * P.sc[0].ref.pitch * sizeof(float), 256);
+    const size_t work = states + sizeof(double) * (z->tile_doubles() + z->out_doubles());
+    const bool shared = one_channel && work <= z->stage_bytes();
+    z->plane_bytes = planes + (shared ? 0 : work);
+    cudaError_t e = cudaMalloc(&z->planes, z->plane_bytes);
+    if (e == cudaSuccess) e = cudaMalloc((void **)&z->stage, z->stage_bytes());
+    if (e != cudaSuccess) {
+        cudaGetLastError();  // not an error of the launches that follow
+        cudaFree(z->planes);
+        z->planes = nullptr;
+        return e;
+    }
+    char *const area = shared ? (char *)z->stage : (char *)z->planes + planes;
+    for (int s = 0; s < P.ns; s++) P.sc[s].state = (float *)(area + (one_channel ? 0 : state[s]));
+    z->tile_out = (double *)(area + states);
+    return cudaSuccess;
+}
 
 s2_status s2_zensim_create(int32_t device, uint32_t width, uint32_t height, s2_zensim **out) {
     return s2_zensim_create_limited(device, width, height, kZsMaxState, out);
@@ -135,15 +162,8 @@ s2_status s2_zensim_create_limited(int32_t device, uint32_t width, uint32_t heig
         n = n / 2;
         h = (h + 1) / 2;
     }
-    const size_t planes = bytes;
-    P.one_channel = states > max_state;
-    if (P.one_channel)
-        states = align_up((size_t)((P.sc[0].h + kZsSub - 1) / kZsSub) * 4 * P.sc[0].ref.pitch * sizeof(float), 256);
-    z->plane_bytes = bytes += states;
-    cudaError_t e = cudaMalloc(&z->planes, bytes);
-    if (e == cudaSuccess) e = cudaMalloc((void **)&z->stage, (size_t)width * 3 * height);
-    if (e == cudaSuccess)
-        e = cudaMalloc((void **)&z->tile_out, sizeof(double) * (z->tile_doubles() + z->out_doubles()));
+    cudaError_t e = zs_allocate(z, bytes, states, state, states > max_state);
+    if (e == cudaErrorMemoryAllocation && !P.one_channel) e = zs_allocate(z, bytes, states, state, true);
     if (e != cudaSuccess) {
         s2_zensim_destroy(z);
         return e == cudaErrorMemoryAllocation ? S2_ERR_OOM : s2_cuda_fail(e, "zensim buffers");
@@ -154,7 +174,6 @@ s2_status s2_zensim_create_limited(int32_t device, uint32_t width, uint32_t heig
         ZsPlanes *pl[2] = {&S.ref, &S.dis};
         for (int img = 0; img < 2; img++)
             for (int c = 0; c < 3; c++) pl[img]->p[c] = (float *)((char *)z->planes + off[s][img] + c * plane) + kZsLeft;
-        S.state = (float *)((char *)z->planes + planes + (P.one_channel ? 0 : state[s]));
     }
     *out = z;
     return S2_OK;
@@ -166,7 +185,6 @@ void s2_zensim_destroy(s2_zensim *z) {
     cudaDeviceSynchronize();
     cudaFree(z->planes);
     cudaFree(z->stage);
-    cudaFree(z->tile_out);
     delete z;
 }
 
@@ -290,8 +308,6 @@ s2_status s2_zensim_raw(const s2_zensim *z, double *acc, uint32_t *peaks) {
 
 s2_status s2_zensim_mem_usage(const s2_zensim *z, size_t *bytes) {
     if (!z || !bytes) return S2_ERR_INVALID_ARG;
-    const size_t b = (size_t)z->w * 3 * z->h + z->plane_bytes +
-                     sizeof(double) * (z->tile_doubles() + z->out_doubles());
-    *bytes = b;
+    *bytes = z->stage_bytes() + z->plane_bytes;
     return S2_OK;
 }
