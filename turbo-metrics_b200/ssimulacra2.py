@@ -63,7 +63,8 @@ def _host_ptr(img, elem_bytes):
     if isinstance(img, np.ndarray):
         if img.strides[-1] != img.itemsize or (img.ndim == 3 and img.strides[1] != img.shape[2] * img.itemsize):
             raise capi.S2Error(capi.S2_ERR_INVALID_ARG, "rows must be packed samples")
-        return img.ctypes.data, img.strides[0]
+        # a flipped view's negative stride as the C field holds it (the upload refuses it)
+        return img.ctypes.data, img.strides[0] & 0xffffffffffffffff
     if img.is_cuda:
         raise capi.S2Error(capi.S2_ERR_INVALID_ARG, "expected a host (CPU) tensor")
     stride = img.stride()
@@ -310,7 +311,10 @@ class PairDesc:
             matrix, range_ = capi.MATRIX[self.matrix], capi.RANGE[self.range]
         if dis_only:
             rp = ru = 0
-        return (shape[1], shape[0], capi.FMT[self.fmt], self.bits, rp, dp, ru, du, rpitch, dpitch, matrix, range_)
+        bits = self.bits
+        if type(bits) is not int or not -0x80000000 <= bits < 0x80000000:
+            bits = ctypes.c_int32(bits).value  # an integer, as a C field takes it: numpy would round and parse
+        return (shape[1], shape[0], capi.FMT[self.fmt], bits, rp, dp, ru, du, rpitch, dpitch, matrix, range_)
 
     def to_c(self, host=False):
         d = capi.PairDescC()
