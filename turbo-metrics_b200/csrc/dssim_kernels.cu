@@ -44,10 +44,8 @@ __host__ __device__ __forceinline__ float ds_k(int i) {
 
 __device__ __forceinline__ int ds_clamp(int v, int hi) { return v < 0 ? 0 : (v > hi ? hi : v); }
 
-// Fixed-order sum of n doubles by the whole block (kDsThreads threads):
-// strided per-thread sums, then a tree; every caller gets the same value for
-// the same array.
-// a thread's share of a fixed-order sum: every 256th value
+// A fixed-order sum of n doubles by a block of kDsThreads threads: each thread's
+// share is every 256th value, then ds_warp_tree adds the shares.
 __device__ double ds_strided_sum(const double *p, int n) {
     double s = 0.0;
     for (int i = threadIdx.x; i < n; i += kDsThreads) s += p[i];
@@ -63,20 +61,6 @@ __device__ double ds_warp_tree(const double *red, int lane) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
     return v;
-}
-
-__device__ double ds_block_reduce(double v, double *red) {
-    const int t = threadIdx.x;
-    __syncthreads();
-    red[t] = v;
-    __syncthreads();
-    for (int w = kDsThreads / 2; w > 0; w >>= 1) {
-        if (t < w) red[t] += red[t + w];
-        __syncthreads();
-    }
-    const double r = red[0];
-    __syncthreads();
-    return r;
 }
 
 __device__ __forceinline__ int ds_find_seg(const DsSeg *segs, int nseg, int tile) {

@@ -7,8 +7,6 @@
 #pragma once
 #include <type_traits>
 
-#include <cuda_bf16.h>
-#include <cuda_fp16.h>
 #include <stdint.h>
 
 namespace s2 {
@@ -378,7 +376,6 @@ __device__ __forceinline__ float2 s2_pfma(float2 a, float2 b, float2 c) {
 
 __device__ __forceinline__ float2 s2_mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ float2 s2_add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
-__device__ __forceinline__ float2 s2_mul2s(float2 a, float2 b) { return make_float2(a.x * b.x, a.y * b.y); }
 
 // The negated quotients -(a.x / b.x, a.y / b.y) by s2_div's steps on both
 // lanes, with the reciprocals of -b: r' = -r, q' = a r' = -q, e = b q' + a =
@@ -496,16 +493,8 @@ struct ColorConsts {
 
 template <typename T> __device__ __forceinline__ float ld_store(const T *p);
 template <> __device__ __forceinline__ float ld_store<float>(const float *p) { return __ldg(p); }
-template <> __device__ __forceinline__ float ld_store<__half>(const __half *p) { return __half2float(*p); }
-template <> __device__ __forceinline__ float ld_store<__nv_bfloat16>(const __nv_bfloat16 *p) {
-    return __bfloat162float(*p);
-}
 template <typename T> __device__ __forceinline__ T to_store(float v);
 template <> __device__ __forceinline__ float to_store<float>(float v) { return v; }
-template <> __device__ __forceinline__ __half to_store<__half>(float v) { return __float2half_rn(v); }
-template <> __device__ __forceinline__ __nv_bfloat16 to_store<__nv_bfloat16>(float v) {
-    return __float2bfloat16_rn(v);
-}
 
 // A 2x2 quad of linear RGB: [row][channel], lanes = left and right pixel.
 struct Quad {

@@ -5,7 +5,7 @@
 //   prep_kernel      reads each pair's scale-0 input once (any input format,
 //                    converted to linear RGB on the fly), builds the 2x2 box
 //                    pyramid in linear RGB and writes the XYB planes of all
-//                    six scales (planar, f32/f16/bf16).
+//                    six scales (planar, f32).
 //                    (ssimulacra2-cuda-kernel/src/downscale.rs:4-35, srgb.rs,
 //                    xyb.rs)
 //   fused_kernel     persistent; each work item is one channel of a tile of
@@ -1112,14 +1112,11 @@ static const double kWeights[108] = {
     0.0, 0.0, 0.0, 0.0005130064588990679, 0.0, 0.00010854057858411537,
 };
 
-const double *host_weights() { return kWeights; }
-
 cudaError_t upload_weights() { return cudaMemcpyToSymbol(c_weight, kWeights, sizeof kWeights); }
 
 size_t fused_smem_bytes() { return (size_t)kBufF2 * sizeof(float2) + (size_t)kStages * kStageFloats * sizeof(float) + 6 * kFusedThreads * sizeof(double); }
 constexpr int kExportBlocks = kTileBlocks - 1;  // resident blocks per SM: the map rows take one block's room
 static size_t export_smem_bytes() { return fused_smem_bytes() + 3 * kExpMap * sizeof(float); }
-int fused_threads() { return kTileThreads; }
 
 template <bool EXPORT>
 static cudaError_t fused_attrs() {

@@ -5,7 +5,6 @@
 #include "ssim2_device.cuh"
 
 namespace s2 {
-const double *host_weights();
 cudaError_t upload_weights();
 cudaError_t configure_kernels();
 size_t fused_smem_bytes();
