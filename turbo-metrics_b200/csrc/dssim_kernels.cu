@@ -515,10 +515,10 @@ __global__ void __launch_bounds__(kDsThreads, kDsBlocks) dssim_tile_kernel(const
 // and 20 multiplies per four outputs, where the tile pass below spends twice
 // that per output on windows that two threads form, shared-memory traffic and
 // 12 % of halo.  16 x 720p pairs (Lab of five levels): 727 us against the tile
-// pass's 962.  A strip is a chain of 40 to 136 dependent rows of about 2 us,
-// so a submission with few strips is faster in tiles (1600x1067: 140 against
-// 124 us): see choose_ds_rows.
-//
+// pass's 962.  A strip is a chain of 72 dependent rows of about 2 us, whatever
+// part of its 120 columns the level fills, so a submission with few strips, or
+// with narrow levels, is faster in tiles (1920x1080: 161 against 192 us for the
+// DSSIM passes, 256 64x64 pairs: 187 against 265): see choose_ds_rows.
 namespace strip {
 
 struct DsRow {

@@ -735,7 +735,9 @@ s2_status s2_error_maps(s2_ctx *ctx, int32_t scale, float *maps, size_t pitch, v
     if (pitch < row || pitch % sizeof(float)) return S2_ERR_DIM_MISMATCH;
     // the last compute's descriptor and XYB planes are still in the workspace;
     // re-run the tile pass over this scale with the export on, in tiles as tall
-    // as leave about four waves of (tile, channel) items, like the planner's
+    // as leave four items (tile, channel) per resident block of the compute's
+    // tile pass, like the planner's (over five per block of the export, which has
+    // three blocks per SM to the compute's four)
     Seg seg = {};
     seg.scale = scale;
     seg.tiles_x = (p.w[scale] + kTileW - 1) / kTileW;

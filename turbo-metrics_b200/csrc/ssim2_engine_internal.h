@@ -193,6 +193,9 @@ struct Engine {
     // Where a submission's results are formed: for a few pairs the page-locked
     // host array itself (the last kernels' stores cross the link, 1.8 KB a
     // pair), which saves the copy behind them; else device memory and one copy.
+    // Copied / direct, us of device time a submission: 1 64x64 pair 35 / 27, 4
+    // 256x256 52 / 45, 8 256x256 69 / 64, 16 512x512 218 / 216: no size up to 64 pairs
+    // was cheaper by the copy; four covers the calls that wait for one result.
     static constexpr int kDirectPairs = 4;
     DevResult *results_at(int n) const { return n <= kDirectPairs ? results_h : (DevResult *)results_d.p; }
     int *err_word() const { return (int *)counter_d.p + kCounterBytes / sizeof(int) - 1; }
@@ -454,7 +457,10 @@ struct Engine {
     // one block's time, and the small form's is shorter; beyond that its blocks
     // run in waves.  sRGB8 pairs on 148 SMs, small against large form: 640x480
     // (80 blocks) 12.9 / 23.2 us, 1280x720 (240) 23.5 / 25.9, 1600x1066 (425)
-    // 39.5 / 30.5, 1920x1080 (510) 45.5 / 37.3.
+    // 39.5 / 30.5, 1920x1080 (510) 45.5 / 37.3.  The line holds for submissions of
+    // one image per pair too, whose other half of the small form's items is passed
+    // over (a whole call): set_reference 640x480 26 / 28, 1280x720 30 / 30, 1920x1080
+    // 43 / 34; candidates 640x480 50 / 53, 1280x720 72 / 72, 2 1000x900 116 / 106.
     int choose_pyr_blk(const s2_pair_desc *d, int n) const {
         uint64_t blocks = 0;
         for (int i = 0; i < n; i++)

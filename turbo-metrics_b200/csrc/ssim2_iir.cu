@@ -24,13 +24,18 @@
 //                          pooling of lib.rs:986-1016 (f64 sums of d and of
 //                          the f32 (d*d)*(d*d)); one partial-sum record per 32 rows.
 //
-// Both walks are chains of one multiply-add per sample (blur.rs: each output
-// needs the two before it), so a line takes its length times that latency
-// whatever the throughput; what there is to do is to keep everything else off
-// the chain.  One 1280x853 pair (B200, each kernel alone, cold): the vertical
-// walk 51 us with its rows copied ahead (505 us with a load per step on the
-// chain), the horizontal walk 90 us (1487 us as a thread per row and channel,
-// whose five planes' loads were uncoalesced, with the maps on the chain).
+// What bounds them: a line is walked by one lane in order, and its warp issues
+// a sample's instructions one after the other, most of them dependent.  Only
+// one multiply-add of them is the recursion itself (about 4 cycles); the loads,
+// products, window sum, three filters and output sum come to about 25 a sample
+// in the vertical walk, issued 4 to 5 cycles apart: 115 cycles.  What was done
+// is to keep memory latency and the maps off that stream.  One 1280x853 pair
+// (B200, each kernel alone, cold): the vertical walk 50 us with its rows copied
+// ahead (505 us with a load per step on the stream), the horizontal walk 91 us
+// (1487 us as a thread per row and channel, whose five planes' loads were
+// uncoalesced, with the maps on the stream): 139 cycles a sample, where the
+// walkers and the helpers wait for one another at a barrier per 32 columns and
+// a little over half of the issue slots are used.
 //
 // The XYB planes come from prep_kernel (same pyramid and XYB arithmetic as the
 // reference, with the engine's own cube root); finalize_kernel reduces the row
@@ -174,7 +179,7 @@ __global__ void __launch_bounds__(kVThreads) iir_vertical_kernel(const DevPair *
 // whose XYB samples they loaded a chunk before; one barrier per chunk.  Both
 // sides are dependent instructions (about one every five cycles a warp): with
 // five helpers, and the copies on the walkers, the pass took 109 us instead
-// of 90 us.
+// of 91 us.
 constexpr int kHc = 32, kHp = kHc + 4, kHSlots = 4;
 constexpr int kHPlane = kHc * kHp;                     // floats of one plane of a chunk
 constexpr int kWalkers = 5, kHelpers = 11;

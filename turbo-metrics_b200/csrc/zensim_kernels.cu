@@ -27,10 +27,10 @@
 // threads and took 2154 us, waiting on its own chain.  Only the four running
 // sums are a chain (two dependent adds per row); with their state saved every
 // 8 rows everything else runs in parallel at the same f32 roundings.  Per
-// 1080p pair now (B200, each kernel alone): prep 20 us per image (49 + 17 us
-// as four launches), walk 73 us (its row loads' latency and the barrier per
+// 1080p pair now (B200, each kernel alone, cold): prep 24 us per image (49 + 17
+// us as four launches), walk 73 us (its row loads' latency and the barrier per
 // chunk), features 104 us (issue: 290 instructions per pixel and channel, of
-// them 96 for the horizontal sums, 17 f64 adds and 17 conversions), reduce 9 us.
+// them 96 for the horizontal sums, 17 f64 adds and 17 conversions), reduce 10 us.
 //
 // Sums are reduced in a fixed order -- where the reference adds each column
 // with a float atomic -- so results do not depend on scheduling.
